@@ -5,14 +5,14 @@ import numpy as np
 import pytest
 
 import luce_render_b200 as lr
-from tests.render_cases import cases
+import render_cases
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("index", range(11))
 def test_forked_pass_equals_serial_pass(index):
-    scene, settings = cases()[index]
+    scene, settings = render_cases.cases()[index]
     ctx = lr.Context(0)
     images = []
     for profile in (0, 1):
