@@ -282,11 +282,12 @@ void launch_shadow(int width, int stack, int block, bool count, bool cutouts, bo
     }
 }
 
-// Lets every kernel of variant (W, kStack) take `bytes` of dynamic shared memory (above
-// the default 48 KB for deep stacks in large blocks).
+// Lets every kernel of variant (W, kStack) take the dynamic shared memory of its stacks at
+// the largest block. The allowance is the kernel's, not a wave's: set for one block size it
+// would refuse the launches of a wave that runs a larger one.
 template <int W, int kStack>
-void allow_stacks(size_t bytes) {
-    const int b = (int)bytes;
+void allow_stacks() {
+    const int b = (int)stack_bytes<W, kStack>(kTraceBlockMax);
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if constexpr (W == 2) LR_CUDA(cudaFuncSetAttribute(closest_bvh2_kernel<kStack>, a, b));
     else LR_CUDA(cudaFuncSetAttribute(closest_kernel<W, kStack, false, false>, a, b));
@@ -308,7 +309,7 @@ int closest_grid(int width, int stack, int block, bool refill, int sm_count) {
 #define LR_CASE(wd, k)                                                                                        \
     case wd * 1000 + k: {                                                                                     \
         const size_t bytes = stack_bytes<wd, k>(block);                                                       \
-        allow_stacks<wd, k>(bytes);                                                                           \
+        allow_stacks<wd, k>();                                                                                \
         if (refill)                                                                                           \
             LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closest_kernel<wd, k, false, true>, block, \
                                                                   bytes));                                    \
