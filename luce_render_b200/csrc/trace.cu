@@ -35,10 +35,11 @@ __device__ __forceinline__ void warp_batches(uint32_t count, uint32_t *next, Bod
 
 // intersect_closest.comp:45-76: the nearest triangle, then the analytic lights
 // before it (camera rays skip lights invisible to the camera). Two ways through the queue,
-// chosen by the plan: warp batches (warp_batches: 32 neighbouring entries a warp at a
-// time), which keep a warp's lanes on similar nodes; with plan refill_at > 0 persistent
-// warps hand finished lanes new entries one by one instead (trace_refilling), which keeps
-// more lanes busy on incoherent rays.
+// chosen by the plan on the wide trees: warp batches (warp_batches: 32 neighbouring entries
+// a warp at a time), which keep a warp's lanes on similar nodes; with plan refill_at > 0
+// persistent warps hand finished lanes new entries one by one instead (trace_refilling),
+// which keeps more lanes busy on incoherent rays. On the BVH2 the queue's length decides:
+// long ones take the voted walk (trace_voted), short ones warp batches.
 template <int W, int kStack, bool kCount, bool kRefill>
 __device__ __forceinline__ void closest_body(const Wave &w, uint32_t round) {
     extern __shared__ int stack[];  // kInts entries a thread, strided by the block's size
@@ -76,7 +77,13 @@ __device__ __forceinline__ void closest_body(const Wave &w, uint32_t round) {
         if (light != kNone) what = kLightHit | light;
         hits[i] = make_float4(t, __uint_as_float(what), tr.h.u, tr.h.v);
     };
-    if (kRefill) {
+    if (W == 2 && long_queue(count)) {
+        if constexpr (W == 2) {
+            DeviceScene s;
+            trace_voted(tr, s, count, fetch_counter(w, round, false), [&](uint32_t j) { return begin(j, s); }, end,
+                        overflow, visits);
+        }
+    } else if (kRefill) {
         auto begin_or_end = [&](uint32_t j, DeviceScene &s) {
             if (begin(j, s)) return true;
             end(j);
@@ -105,14 +112,8 @@ __global__ void __launch_bounds__(kTraceBlockMax, kTraceMinBlocks) closest_kerne
     closest_body<W, kStack, kCount, kRefill>(w, round);
 }
 
-// The BVH2's grid-stride walk, the renderer's default, at 56 registers: nine blocks of 128
-// threads an SM instead of eight, for the latency of its dependent node fetches (8 bytes
-// spilled outside the walk). Measured on the headline pass over several boxes: 1,225-1,237
-// Mrays/s against 1,214-1,225 at 64 registers -- about 1 %, within what boxes differ by.
-template <int kStack>
-__global__ void __maxnreg__(56) closest_bvh2_kernel(Wave w, uint32_t round) {
-    closest_body<2, kStack, false, false>(w, round);
-}
+// A shadow ray's hit id when its connection ended before the any-hit walk.
+constexpr int kNothingTraced = -2;
 
 // intersect_shadow.comp:28-92: unblocked light samples join their path's radiance; a light
 // path's camera connection, unless a light the camera sees stands in it, splats its value
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kTraceBlockMax, kCutouts ? 1 : kTraceMinBlocks
         return !(w.plan->seg[tag >> kPathBits].kind == kLightSegment && seen_light_between(m.lights, xyz(o), xyz(d), d.w));
     };
     auto end = [&](uint32_t i) {
+        if (tr.h.id == kNothingTraced) return;
         const bool blocked = tr.h.id >= 0;
         record(i, blocked ? 1.0f : 0.0f);
         if (!blocked) deliver(i, 1.0f, false);
@@ -213,7 +215,19 @@ __global__ void __launch_bounds__(kTraceBlockMax, kCutouts ? 1 : kTraceMinBlocks
         }
         if (through) deliver(i, kept, true);
     };
-    if (kRefill && !kCutouts) {
+    if (W == 2 && !kCutouts && long_queue(count)) {
+        if constexpr (W == 2) {
+            DeviceScene s;
+            auto begin_voted = [&](uint32_t i) {
+                tr.h.id = kNothingTraced;
+                if (!prologue(i)) return false;
+                const float4 o = w.shadow_o[i], d = w.shadow_d[i];
+                s = member_of(__float_as_uint(o.w)).scene;
+                return tr.start(s, Ray{xyz(o), 0.0f, xyz(d), d.w});
+            };
+            trace_voted(tr, s, count, fetch_counter(w, round, true), begin_voted, end, overflow, visits);
+        }
+    } else if (kRefill && !kCutouts) {
         trace_refilling(tr, count, fetch_counter(w, round, true), w.plan->head.refill_at, begin, end, overflow, visits);
     } else {
         warp_batches(count, fetch_counter(w, round, true), [&](uint32_t i) {
@@ -252,8 +266,8 @@ void launch_closest(int width, int stack, int block, bool count, bool refill, in
     case wd * 1000 + k: {                                                                           \
         const size_t bytes = stack_bytes<wd, k>(block);                                             \
         if (count) closest_kernel<wd, k, true, false><<<grid, block, bytes, stream>>>(w, round);    \
-        else if (refill) closest_kernel<wd, k, false, true><<<grid, block, bytes, stream>>>(w, round); \
-        else if constexpr (wd == 2) closest_bvh2_kernel<k><<<grid, block, bytes, stream>>>(w, round); \
+        else if (refill && wd != 2)                                                                 \
+            closest_kernel<wd, k, false, wd != 2><<<grid, block, bytes, stream>>>(w, round);        \
         else closest_kernel<wd, k, false, false><<<grid, block, bytes, stream>>>(w, round);         \
         return;                                                                                     \
     }
@@ -272,7 +286,8 @@ void launch_shadow(int width, int stack, int block, bool count, bool cutouts, bo
         if (count && cutouts) shadow_kernel<wd, k, true, true, false><<<grid, block, bytes, stream>>>(w, round);   \
         else if (count) shadow_kernel<wd, k, true, false, false><<<grid, block, bytes, stream>>>(w, round);        \
         else if (cutouts) shadow_kernel<wd, k, false, true, false><<<grid, block, bytes, stream>>>(w, round);      \
-        else if (refill) shadow_kernel<wd, k, false, false, true><<<grid, block, bytes, stream>>>(w, round);       \
+        else if (refill && wd != 2)                                                                           \
+            shadow_kernel<wd, k, false, false, wd != 2><<<grid, block, bytes, stream>>>(w, round);            \
         else shadow_kernel<wd, k, false, false, false><<<grid, block, bytes, stream>>>(w, round);                  \
         return;                                                                                               \
     }
@@ -289,12 +304,13 @@ template <int W, int kStack>
 void allow_stacks() {
     const int b = (int)stack_bytes<W, kStack>(kTraceBlockMax);
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if constexpr (W == 2) LR_CUDA(cudaFuncSetAttribute(closest_bvh2_kernel<kStack>, a, b));
-    else LR_CUDA(cudaFuncSetAttribute(closest_kernel<W, kStack, false, false>, a, b));
-    LR_CUDA(cudaFuncSetAttribute(closest_kernel<W, kStack, false, true>, a, b));
+    LR_CUDA(cudaFuncSetAttribute(closest_kernel<W, kStack, false, false>, a, b));
+    if constexpr (W != 2) {
+        LR_CUDA(cudaFuncSetAttribute(closest_kernel<W, kStack, false, true>, a, b));
+        LR_CUDA(cudaFuncSetAttribute(shadow_kernel<W, kStack, false, false, true>, a, b));
+    }
     LR_CUDA(cudaFuncSetAttribute(closest_kernel<W, kStack, true, false>, a, b));
     LR_CUDA(cudaFuncSetAttribute(shadow_kernel<W, kStack, false, false, false>, a, b));
-    LR_CUDA(cudaFuncSetAttribute(shadow_kernel<W, kStack, false, false, true>, a, b));
     LR_CUDA(cudaFuncSetAttribute(shadow_kernel<W, kStack, false, true, false>, a, b));
     LR_CUDA(cudaFuncSetAttribute(shadow_kernel<W, kStack, true, false, false>, a, b));
     LR_CUDA(cudaFuncSetAttribute(shadow_kernel<W, kStack, true, true, false>, a, b));
@@ -310,11 +326,9 @@ int closest_grid(int width, int stack, int block, bool refill, int sm_count) {
     case wd * 1000 + k: {                                                                                     \
         const size_t bytes = stack_bytes<wd, k>(block);                                                       \
         allow_stacks<wd, k>();                                                                                \
-        if (refill)                                                                                           \
-            LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closest_kernel<wd, k, false, true>, block, \
+        if (refill && wd != 2)                                                                                \
+            LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closest_kernel<wd, k, false, wd != 2>, block, \
                                                                   bytes));                                    \
-        else if constexpr (wd == 2)                                                                           \
-            LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closest_bvh2_kernel<k>, block, bytes)); \
         else                                                                                                  \
             LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closest_kernel<wd, k, false, false>, block, \
                                                                   bytes));                                    \

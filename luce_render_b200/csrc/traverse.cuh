@@ -42,6 +42,15 @@ struct Hit {
 __device__ __forceinline__ float fmul_(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fadd_(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub_(float a, float b) { return __fsub_rn(a, b); }
+// 32 bytes, 32-byte aligned, in one load instruction. A warp's lanes walk different nodes, and
+// L1 looks up one line a lane for every load instruction, so half as many loads a node is
+// half the lookups.
+__device__ __forceinline__ void ldg32(const float4 *p, float4 &a, float4 &b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
 __device__ __forceinline__ float comp(const float3 &v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
 // bvh.glsl:55-56: components below 1e-20 in magnitude become +-1e-20 (+ for zero).
@@ -256,30 +265,36 @@ struct ExactTracer {
                          r.tmin, r.tmax, enter);
     }
 
-    // Interior visits until a leaf, then that leaf. True when the ray is done.
-    __device__ __forceinline__ bool step(const DeviceScene &s, bool &overflow, Visits &visits) {
-        const DeviceBvh &b = s.bvh;
-        while (node >= 0) {
-            if (kCount) visits.nodes++;
-            const float4 *e = b.entries + (size_t)node * 4;
-            const float4 n0 = __ldg(e), n1 = __ldg(e + 1), n2 = __ldg(e + 2), n3 = __ldg(e + 3);
-            float ea, eb;
-            const bool ha = box_exact(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, inv, oinv, r.tmin, h.t, ea);
-            const bool hb = box_exact(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, inv, oinv, r.tmin, h.t, eb);
-            const int l0 = __float_as_int(n3.x), l1 = __float_as_int(n3.y);
-            if (ha && hb) {
-                const bool left_first = ea <= eb;
-                if (!st.push(left_first ? l1 : l0)) overflow = true;
-                node = left_first ? l0 : l1;
-            } else if (ha) {
-                node = l0;
-            } else if (hb) {
-                node = l1;
-            } else {
-                if (st.empty()) return true;
-                node = st.pop();
-            }
+    // One interior visit (node >= 0): on to the nearer hit child, or a waiting subtree. True
+    // when the ray is done.
+    __device__ __forceinline__ bool visit(const DeviceScene &s, bool &overflow, Visits &visits) {
+        if (kCount) visits.nodes++;
+        const float4 *e = s.bvh.entries + (size_t)node * 4;
+        float4 n0, n1, n2, n3;
+        ldg32(e, n0, n1);
+        ldg32(e + 2, n2, n3);
+        float ea, eb;
+        const bool ha = box_exact(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, inv, oinv, r.tmin, h.t, ea);
+        const bool hb = box_exact(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, inv, oinv, r.tmin, h.t, eb);
+        const int l0 = __float_as_int(n3.x), l1 = __float_as_int(n3.y);
+        if (ha && hb) {
+            const bool left_first = ea <= eb;
+            if (!st.push(left_first ? l1 : l0)) overflow = true;
+            node = left_first ? l0 : l1;
+        } else if (ha) {
+            node = l0;
+        } else if (hb) {
+            node = l1;
+        } else {
+            if (st.empty()) return true;
+            node = st.pop();
         }
+        return false;
+    }
+
+    // The leaf in hand (node < 0): its triangles, then a waiting subtree. True when the ray is
+    // done.
+    __device__ __forceinline__ bool leaf(const DeviceScene &s, Visits &visits) {
         uint32_t first, count;
         leaf_range(node, first, count);
         if (kCount) visits.tests += count;
@@ -302,6 +317,13 @@ struct ExactTracer {
         if (st.empty()) return true;
         node = st.pop();
         return false;
+    }
+
+    // Interior visits until a leaf, then that leaf. True when the ray is done.
+    __device__ __forceinline__ bool step(const DeviceScene &s, bool &overflow, Visits &visits) {
+        while (node >= 0)
+            if (visit(s, overflow, visits)) return true;
+        return leaf(s, visits);
     }
 };
 
@@ -521,8 +543,10 @@ struct CompressedTracer {
     // order for this direction) and `more` the ranks of the other hit children, one bit
     // each (0: none).
     __device__ __forceinline__ bool visit(const float4 *n, int &next, uint32_t &more) {
-        const float4 head = __ldg(n), la = __ldg(n + 1), lb = __ldg(n + 2), px = __ldg(n + 3), py = __ldg(n + 4),
-                     pz = __ldg(n + 5);
+        float4 head, la, lb, px, py, pz;
+        ldg32(n, head, la);
+        ldg32(n + 2, lb, px);
+        ldg32(n + 4, py, pz);
         const uint32_t meta = __float_as_uint(head.w);
         const float ax = q_step(meta & 0xffu) * inv.x, ay = q_step((meta >> 8) & 0xffu) * inv.y,
                     az = q_step((meta >> 16) & 0xffu) * inv.z;
@@ -656,15 +680,92 @@ struct TracerOf<2, kAny, kStack, kCount> {
     static constexpr int kInts = kStack;
 };
 
+// The BVH2 walk of a long queue: a warp votes each step between nodes and leaves, and refills.
+//
+// Walked ray by ray (trace_batched), a warp's lanes wait twice: in the node loop until the
+// last lane has reached a leaf, and at the end until the longest of 32 rays is done. On
+// incoherent rays 7 of 32 lanes work while the issue slots are 74 % busy, so the walk is
+// bound by instructions issued for idle lanes. Here
+//   - all lanes step through nodes as long as kVoteNodes of them stand at one; the others,
+//     at a leaf, wait for no more than that, then every lane at a leaf tests it;
+//   - once kVoteRefill lanes have finished their rays they finish them together (`end`) and
+//     take the queue's next entries with one atomic (`begin`).
+// A ray's own order of visits does not change, so neither does any answer, any-hit ids
+// included. Measured (B200, 1M triangles): 4,194,304 incoherent rays 1,863 -> 1,389 us,
+// the 1080p pass's first bounce (1,049,661 rays) 723 -> 531, its first shadow rays (555,285)
+// 438 -> 325, its primary rays 581 -> 522; the whole pass (4 samples, image read) 13.09 -> 11.72
+// ms, at 64 registers (12.23 at 56, which spills). Votes at 16, 12, 8, 4 and 1 lanes: 1,384, 1,387,
+// 1,409, 1,503 and 1,700 us on the incoherent rays with refills at 8 lanes, but 99, 91, 89, 87
+// and 89 on the glossy box's 256,000 (leaves outnumber nodes there); refills at 8, 16, 24
+// and 32 lanes with the vote at 8: 1,409, 1,389, 1,442, 1,968.
+//
+// The loop stays converged around its ballots and ends: a pass of it steps every ray in
+// hand at least once along a finite tree. `s` is the scene of this lane's ray; `begin(i)` sets
+// it up and starts ray i, false when there is no walk to take.
+constexpr int kVoteNodes = 8, kVoteRefill = 16;
+constexpr int kIdleLane = (int)0x80000000;  // a lane's node between rays: no leaf link is that low
+
+template <class Tracer, class Begin, class End>
+__device__ __forceinline__ void trace_voted(Tracer &tr, const DeviceScene &s, uint32_t count, uint32_t *next,
+                                            Begin begin, End end, bool &overflow, Visits &visits) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t i = 0;
+    bool ended = true, drained = false;
+    tr.node = kIdleLane;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, tr.node == kIdleLane);
+        const bool last = drained && idle == 0xffffffffu;
+        if (last || (!drained && __popc(idle) >= kVoteRefill)) {
+            if (tr.node == kIdleLane && !ended) {
+                end(i);
+                ended = true;
+            }
+            if (last) break;
+            const uint32_t want = (uint32_t)__popc(idle);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(next, want);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            drained = base + want >= count;
+            if (tr.node == kIdleLane) {
+                i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+                if (i < count) {
+                    ended = false;
+                    if (!begin(i)) tr.node = kIdleLane;
+                }
+            }
+            __syncwarp();
+        }
+        do {
+            if (tr.node >= 0 && tr.visit(s, overflow, visits)) tr.node = kIdleLane;
+        } while (__popc(__ballot_sync(0xffffffffu, tr.node >= 0)) >= kVoteNodes);
+        if (tr.node < 0 && tr.node != kIdleLane && tr.leaf(s, visits)) tr.node = kIdleLane;
+        __syncwarp();
+    }
+}
+
+// Whether a queue of `count` rays is long enough for the voted walk: more rays than the
+// launch has lanes, so that finished lanes have rays to take. Shorter queues are bound by
+// their longest rays, which the plain walk takes with less bookkeeping (glossy box, 171,957
+// rays on 170,496 lanes: 97 us plain, 113 voted; 275,175 rays of a 100k-triangle view: 172 and
+// 148).
+__device__ __forceinline__ bool long_queue(uint32_t count) { return count > gridDim.x * blockDim.x; }
+
 // A resident grid over a queue of `count` rays in warp batches: each warp takes the next
 // 32 consecutive entries (neighbouring primary rays keep its lanes on similar nodes) with
 // one atomic on `next` (zero at launch) whenever its lanes are done, so warps that drew
-// long rays take fewer batches. `load(i)` gives ray i and `store(i, hit, ray)` takes its
+// long rays take fewer batches; a long queue on the BVH2 takes the voted walk. `load(i)` gives ray i and `store(i, hit, ray)` takes its
 // result.
 template <int W, bool kAny, int kStack, bool kCount, class Load, class Store>
 __device__ __forceinline__ void trace_batched(const DeviceScene &s, uint32_t count, uint32_t *next, int *stack_base,
                                               int stride, Load load, Store store, bool &overflow, Visits &visits) {
     typename TracerOf<W, kAny, kStack, kCount>::type tr(stack_base, stride);
+    if constexpr (W == 2) {
+        if (long_queue(count)) {
+            trace_voted(tr, s, count, next, [&](uint32_t i) { return tr.start(s, load(i)); },
+                        [&](uint32_t i) { store(i, tr.h, tr.r); }, overflow, visits);
+            return;
+        }
+    }
     const uint32_t lane = threadIdx.x & 31u;
     for (;;) {
         uint32_t base = 0;
@@ -752,7 +853,9 @@ __device__ __forceinline__ Hit trace_reference(const DeviceScene &s, const Ray &
         } else {
             if (kCount) visits.nodes++;
             const float4 *e = b.entries + (size_t)node * 4;
-            const float4 n0 = __ldg(e), n1 = __ldg(e + 1), n2 = __ldg(e + 2), n3 = __ldg(e + 3);
+            float4 n0, n1, n2, n3;
+            ldg32(e, n0, n1);
+            ldg32(e + 2, n2, n3);
             const float tl = kAny ? r.tmax : h.t;
             const float a = box_reference(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, r.o, inv, tl);
             const float bb = box_reference(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, r.o, inv, tl);
