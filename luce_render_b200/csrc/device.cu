@@ -11,6 +11,7 @@
 
 #include "device.hpp"
 #include "traverse.cuh"
+#include "warpwalk.cuh"
 #include "wide.hpp"
 
 namespace lr {
@@ -23,6 +24,8 @@ namespace {
 constexpr int kBlock = 128;
 // Where the ray queries' batch cursor sits among a context's status words (in ints).
 constexpr int kBatchCursor = 8;
+// Words of stack a warp of a short query has: an 8-wide tree of 32 levels.
+constexpr uint32_t kWarpQueryInts = warp_stack_ints(32);
 
 struct ProbeFrame {
     float b[16];
@@ -106,6 +109,21 @@ __global__ void __launch_bounds__(kBlock) trace_resident_kernel(DeviceScene s, c
     if (kCount) add_visits(counts, visits);
 }
 
+// Closest hits of a short ray list, a warp a ray (warpwalk.cuh). An any-hit query reports the
+// hit it finds first, which is the BVH2 walk's, and does not come here.
+__global__ void __launch_bounds__(kBlock) trace_warps_kernel(DeviceScene s, const float4 *__restrict__ rays, uint32_t n,
+                                                            float4 *__restrict__ hits, int *status, uint32_t *next) {
+    __shared__ int stack[kBlock / 32][kWarpQueryInts];
+    bool overflow = false;
+    warp_rays(n, next, [&](uint32_t i) {
+        const float4 a = __ldg(&rays[2 * (size_t)i]), b = __ldg(&rays[2 * (size_t)i + 1]);
+        const Ray r{make_float3(a.x, a.y, a.z), a.w, make_float3(b.x, b.y, b.z), b.w};
+        const Hit h = walk_warp<false>(s, r, stack[threadIdx.x >> 5], kWarpQueryInts, overflow);
+        if ((threadIdx.x & 31u) == 0u) hits[i] = make_float4(h.t, __int_as_float(h.id), h.u, h.v);
+    });
+    note_overflow(status, overflow);
+}
+
 // Does nothing (the sink is never written): launch-overhead measurements.
 __global__ void idle_kernel(int *sink) {
     if (sink && threadIdx.x == 1023u) *sink = 0;
@@ -166,11 +184,38 @@ void launch_resident(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, flo
                                                                                status, counts, next);
 }
 
+// The resident blocks of the warp-walk kernel on the current device.
+unsigned warps_resident() {
+    static int resident = 0;
+    if (!resident) {
+        int per_sm = 0, device = 0, sms = 0;
+        LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_warps_kernel, kBlock, 0));
+        LR_CUDA(cudaGetDevice(&device));
+        LR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        resident = std::max(1, per_sm) * sms;
+    }
+    return (unsigned)resident;
+}
+
+// Short closest-hit queries of the default width a warp a ray: at most kWarpRays rays a
+// resident warp, on a scene whose 8-wide tree fits the stack.
+bool launch_warps(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, float4 *hits, int *status, cudaStream_t stream) {
+    constexpr uint64_t kWarps = kBlock / 32;
+    const unsigned resident = warps_resident();
+    if (n > kWarpRays * kWarps * (uint64_t)resident || !warp_walkable(gs->scene, kWarpQueryInts)) return false;
+    uint32_t *next = (uint32_t *)(status + kBatchCursor);
+    LR_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + kWarps - 1) / kWarps, resident);
+    trace_warps_kernel<<<grid, kBlock, 0, stream>>>(gs->scene, rays, (uint32_t)n, hits, status, next);
+    return true;
+}
+
 template <bool kAny, bool kCount>
 void dispatch_exact(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, float4 *hits, int *status,
                     unsigned long long *counts, cudaStream_t stream, int requested_width) {
     if (n > 0xffffffffull) fail(LR_LIMIT, "a ray query holds at most 2^32 - 1 rays");
     const TraversalChoice c = choose_traversal(gs->scene, requested_width);
+    if (!kAny && !kCount && requested_width == 0 && c.width == 2 && launch_warps(gs, rays, n, hits, status, stream)) return;
     switch (c.width * 1000 + c.stack) {
         case 8016: launch_resident<8, kAny, 16, kCount>(gs, rays, n, hits, status, counts, stream); break;
         case 8032: launch_resident<8, kAny, 32, kCount>(gs, rays, n, hits, status, counts, stream); break;
@@ -538,6 +583,7 @@ int lr_gpu_scene_upload(lr_context *ctx, const lr_scene *scene, lr_gpu_scene **o
             {sources8.data(), sources8.size() * sizeof(uint32_t), 0},
             {scene->flat.data(), scene->flat.size(), 0},
             {root_box, sizeof root_box, 0},
+            {nullptr, w8.node_count * 16 * sizeof(float4), 0},  // the 8-wide tree's plain boxes
         };
         size_t total = 0;
         for (auto &p : parts) {
@@ -565,6 +611,7 @@ int lr_gpu_scene_upload(lr_context *ctx, const lr_scene *scene, lr_gpu_scene **o
         s.shading = (const uint4 *)(base + parts[7].offset);
         s.wide4 = DeviceWide{(const float4 *)(base + parts[8].offset), T ? 4 : 0, w4.max_stack, w4.node_count};
         s.wide8 = DeviceWide{(const float4 *)(base + parts[9].offset), T ? 8 : 0, w8.max_stack, w8.node_count};
+        s.wide8.boxes = T ? (const float4 *)(base + parts[16].offset) : nullptr;
         gs->wide4_nodes = w4.node_count;
         gs->wide8_nodes = w8.node_count;
         gs->parents = (uint32_t *)(base + parts[10].offset);
@@ -592,6 +639,8 @@ int lr_gpu_scene_upload(lr_context *ctx, const lr_scene *scene, lr_gpu_scene **o
         s.entry_count = L.entries.size() / 4;
         s.depth = scene->bvh_depth;
         stack_for(s.depth);
+        fill_wide_boxes(gs.get(), L.delta, ctx->stream);
+        LR_CUDA(cudaStreamSynchronize(ctx->stream));
         *out = gs.release();
     });
 }

@@ -38,6 +38,9 @@ struct DeviceWide {
     int width = 0;
     uint32_t max_stack = 0;   // the most stack entries a traversal can hold
     uint64_t node_count = 0;
+    // The 8-wide tree's boxes as warps walk them (warpwalk.cuh): 16 float4 a node, two a child
+    // slot -- the widened low corner and the link, the high corner and 1 (0: an empty slot).
+    const float4 *boxes = nullptr;
 };
 
 // A scene in HBM (GpuScene, device.lucb:16-38).
@@ -102,6 +105,8 @@ constexpr uint32_t kRefitRoot = 0xfffffffeu;
 // refit.cu: with the uploaded scene's points already moved (its `positions` array),
 // refits its triangle records, flat normals and every BVH's boxes on `stream`; waits.
 void refit_scene(lr_gpu_scene *gs, cudaStream_t stream);
+// The 8-wide tree's DeviceWide::boxes from the exact BVH2 boxes, widened by `delta`.
+void fill_wide_boxes(lr_gpu_scene *gs, float delta, cudaStream_t stream);
 // FNV-1a over a scene's triangle count and leaf-order indices.
 uint64_t topology_hash(const Scene &scene);
 }  // namespace lr

@@ -39,6 +39,7 @@
 #include "paths.cuh"
 #include "shading.cuh"
 #include "traverse.cuh"
+#include "warpwalk.cuh"
 #include "wave.cuh"
 
 namespace lr {
@@ -1643,11 +1644,25 @@ bool launch_pass(WaveHost *h, bool dry = false, int only = -1) {
             thin = std::max(thin, code);
         }
     }
+    // The scene most of the pass's paths see decides how long BVH2 queues are walked.
+    uint64_t most_triangles = 0;
+    for (uint32_t k = 0, most = 0; k < n; k++)
+        if (seg[k].count > most) {
+            most = seg[k].count;
+            most_triangles = h->members[seg[k].member].dev.scene.triangle_count;
+        }
+    // Short queues a warp a ray, where every member's 8-wide tree fits the stack a warp has in
+    // each of the pass's variants.
+    uint32_t ints = warp_walk_ints(width, stack);
+    if (thin) ints = std::min(ints, warp_walk_ints(8, thin == 1 ? 16 : 32));
+    const bool walkable = std::all_of(rec.members.begin(), rec.members.end(), [&](const std::pair<uint32_t, bool> &e) {
+        return warp_walkable(h->members[e.first].dev.scene, ints);
+    });
     const int variant = width * 1000 + stack + (tracing ? kTracingVariant : 0) + (glossy ? kGlossyVariant : 0) +
                         (cutouts ? kCutoutVariant : 0) + block_index * kBlockVariant +
                         (h->refill_at ? kRefillVariant : 0) + thin * kThinVariant;
     staging->head = PlanHeader{n, used, converts, dry ? 1u : 0u, camera_paths, folds, adapts, h->bin_interval,
-                               h->refill_at, {0u, 0u, 0u}};
+                               h->refill_at, walkable ? kWarpRays : 0u, vote_quarters(most_triangles), 0u};
     staging->display = PlanDisplay{0ull, h->display_scale, h->display_view, 0u, 0u};
     if (h->display_block && converts > 0) {
         rec.display_slot = free_display_slot(h);
@@ -1711,7 +1726,7 @@ void launch_convert(WaveHost *h) {
     rec.number = h->recorded;
     rec.members.push_back({0u, false});
     rec.generations.push_back(mh.generation);
-    staging->head = PlanHeader{0u, 0u, 1u, 0u, 0u, 0u, 0u, 0u, 0u, {0u, 0u, 0u}};
+    staging->head = PlanHeader{0u, 0u, 1u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
     staging->convert[0] = 0u;
     staging->convert_samples[0] = mh.sample;
     rec.display_slot = free_display_slot(h);

@@ -13,8 +13,9 @@
 //      thread waiting on another;
 //   3. the watertight path's widened boxes from the exact ones, with the widening taken
 //      again from the new root box (2^-16 of the scene's scale, one more float step);
-//   4. the 4-wide collapse's child boxes, copied from the BVH2 slots they came from, and the
-//      compressed 8-wide nodes quantized again from those boxes (quantize.hpp).
+//   4. the 4-wide collapse's child boxes, copied from the BVH2 slots they came from, the
+//      compressed 8-wide nodes quantized again from those boxes (quantize.hpp), and the
+//      8-wide tree's plain boxes (DeviceWide::boxes).
 // With the points unchanged a refit leaves every array bit for bit as the upload made it,
 // and the boxes equal the host refit (lr_scene_move_points) of the same move exactly: boxes
 // are minima and maxima of the same floats, and the widening is the same float arithmetic.
@@ -251,6 +252,32 @@ __global__ void quantize_kernel(uint64_t count, const uint32_t *sources, const f
     }
 }
 
+// DeviceWide::boxes: a thread a child slot, its box from the BVH2 slot (or the root) it was
+// collapsed from, its link from the compressed node.
+__global__ void wide_boxes_kernel(uint64_t slots, const uint32_t *sources, const float4 *exact, const float *root_box,
+                                  float delta, const float4 *nodes, float4 *boxes) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < slots; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t source = __ldg(&sources[i]);
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+        if (source != 0xffffffffu) {
+            Box b;
+            if (source == kRefitRoot) {
+                for (int k = 0; k < 3; k++) {
+                    b.lo[k] = root_box[k];
+                    b.hi[k] = root_box[4 + k];
+                }
+            } else {
+                b = read_side(exact, source >> 1, source & 1u);
+            }
+            const float link = __ldg(reinterpret_cast<const float *>(nodes + (i >> 3) * kQNodeFloat4s + 1) + (i & 7u));
+            lo = make_float4(widen_lo(b.lo[0], delta), widen_lo(b.lo[1], delta), widen_lo(b.lo[2], delta), link);
+            hi = make_float4(widen_hi(b.hi[0], delta), widen_hi(b.hi[1], delta), widen_hi(b.hi[2], delta), 1.0f);
+        }
+        boxes[2 * i] = lo;
+        boxes[2 * i + 1] = hi;
+    }
+}
+
 unsigned grid_for(uint64_t items, int sm_count) {
     const uint64_t blocks = (items + 255) / 256;
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)sm_count * 8));
@@ -271,6 +298,15 @@ uint64_t topology_hash(const Scene &scene) {
     mix(counts, sizeof counts);
     mix(scene.indices.data(), scene.indices.size() * sizeof(uint32_t));
     return key;
+}
+
+void fill_wide_boxes(lr_gpu_scene *gs, float delta, cudaStream_t stream) {
+    const DeviceScene &s = gs->scene;
+    if (!s.wide8.boxes) return;
+    wide_boxes_kernel<<<grid_for(gs->wide8_nodes * 8, gs->ctx->sm_count), 256, 0, stream>>>(
+        gs->wide8_nodes * 8, gs->wide8_sources, s.ref_bvh.entries, gs->root_box, delta, s.wide8.nodes,
+        const_cast<float4 *>(s.wide8.boxes));
+    LR_CUDA(cudaGetLastError());
 }
 
 void refit_scene(lr_gpu_scene *gs, cudaStream_t stream) {
@@ -319,6 +355,7 @@ void refit_scene(lr_gpu_scene *gs, cudaStream_t stream) {
     if (s.wide8.width)
         quantize_kernel<<<grid_for(gs->wide8_nodes, sms), 256, 0, stream>>>(
             gs->wide8_nodes, gs->wide8_sources, exact, gs->root_box, delta, const_cast<float4 *>(s.wide8.nodes));
+    fill_wide_boxes(gs, delta, stream);
     LR_CUDA(cudaGetLastError());
     LR_CUDA(cudaStreamSynchronize(stream));
     gs->refits++;

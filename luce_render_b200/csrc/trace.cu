@@ -11,6 +11,7 @@
 #include "device.hpp"
 #include "emitters.cuh"
 #include "traverse.cuh"
+#include "warpwalk.cuh"
 #include "wave.cuh"
 
 namespace lr {
@@ -33,13 +34,24 @@ __device__ __forceinline__ void warp_batches(uint32_t count, uint32_t *next, Bod
     }
 }
 
+// Whether a queue is short enough for a warp a ray: the plan's rays a warp of the launch.
+__device__ __forceinline__ bool short_queue(const Wave &w, uint32_t count) {
+    return count <= w.plan->head.warp_rays * (gridDim.x * (blockDim.x >> 5));
+}
+// The traversal variants that can take the warp walk, and a warp's words of stack in them.
+template <int W, bool kCount>
+constexpr bool kWarpWalk = (W == 2 || W == 8) && !kCount;
+template <int W, int kStack>
+constexpr uint32_t kWarpInts = TracerOf<W, false, kStack, false>::kInts * 32u;
+
 // intersect_closest.comp:45-76: the nearest triangle, then the analytic lights
 // before it (camera rays skip lights invisible to the camera). Two ways through the queue,
 // chosen by the plan on the wide trees: warp batches (warp_batches: 32 neighbouring entries
 // a warp at a time), which keep a warp's lanes on similar nodes; with plan refill_at > 0
 // persistent warps hand finished lanes new entries one by one instead (trace_refilling),
-// which keeps more lanes busy on incoherent rays. On the BVH2 the queue's length decides:
-// long ones take the voted walk (trace_voted), short ones warp batches.
+// which keeps more lanes busy on incoherent rays. On the BVH2 the queue's length and the
+// batch's rays decide (trace_bvh2). The shortest queues, on the BVH2 and the 8-wide tree, take
+// a warp a ray (walk_warp).
 template <int W, int kStack, bool kCount, bool kRefill>
 __device__ __forceinline__ void closest_body(const Wave &w, uint32_t round) {
     extern __shared__ int stack[];  // kInts entries a thread, strided by the block's size
@@ -77,11 +89,21 @@ __device__ __forceinline__ void closest_body(const Wave &w, uint32_t round) {
         if (light != kNone) what = kLightHit | light;
         hits[i] = make_float4(t, __uint_as_float(what), tr.h.u, tr.h.v);
     };
-    if (W == 2 && long_queue(count)) {
+    if (kWarpWalk<W, kCount> && short_queue(w, count)) {
+        int *mine = stack + (threadIdx.x >> 5) * kWarpInts<W, kStack>;
+        warp_rays(count, fetch_counter(w, round, false), [&](uint32_t j) {
+            const uint32_t i = entry(j);
+            const float4 o = ray_o[i], d = ray_d[i];
+            const DeviceScene s = w.members[w.plan->seg[__float_as_uint(o.w) >> kPathBits].member].scene;
+            tr.h = walk_warp<false>(s, Ray{xyz(o), 0.0f, xyz(d), d.w}, mine, kWarpInts<W, kStack>, overflow);
+            if ((threadIdx.x & 31u) == 0u) end(j);
+            __syncwarp();
+        });
+    } else if (W == 2) {
         if constexpr (W == 2) {
             DeviceScene s;
-            trace_voted(tr, s, count, fetch_counter(w, round, false), [&](uint32_t j) { return begin(j, s); }, end,
-                        overflow, visits);
+            trace_bvh2(tr, s, count, fetch_counter(w, round, false), w.plan->head.vote_quarters,
+                       [&](uint32_t j) { return begin(j, s); }, end, overflow, visits);
         }
     } else if (kRefill) {
         auto begin_or_end = [&](uint32_t j, DeviceScene &s) {
@@ -215,17 +237,28 @@ __global__ void __launch_bounds__(kTraceBlockMax, kCutouts ? 1 : kTraceMinBlocks
         }
         if (through) deliver(i, kept, true);
     };
-    if (W == 2 && !kCutouts && long_queue(count)) {
+    if (kWarpWalk<W, kCount> && !kCutouts && short_queue(w, count)) {
+        int *mine = stack + (threadIdx.x >> 5) * kWarpInts<W, kStack>;
+        warp_rays(count, fetch_counter(w, round, true), [&](uint32_t i) {
+            if (!prologue(i)) return;
+            const float4 o = w.shadow_o[i], d = w.shadow_d[i];
+            const DeviceScene s = member_of(__float_as_uint(o.w)).scene;
+            tr.h = walk_warp<true>(s, Ray{xyz(o), 0.0f, xyz(d), d.w}, mine, kWarpInts<W, kStack>, overflow);
+            if ((threadIdx.x & 31u) == 0u) end(i);
+            __syncwarp();
+        });
+    } else if (W == 2 && !kCutouts) {
         if constexpr (W == 2) {
             DeviceScene s;
-            auto begin_voted = [&](uint32_t i) {
+            auto begin_bvh2 = [&](uint32_t i) {
                 tr.h.id = kNothingTraced;
                 if (!prologue(i)) return false;
                 const float4 o = w.shadow_o[i], d = w.shadow_d[i];
                 s = member_of(__float_as_uint(o.w)).scene;
                 return tr.start(s, Ray{xyz(o), 0.0f, xyz(d), d.w});
             };
-            trace_voted(tr, s, count, fetch_counter(w, round, true), begin_voted, end, overflow, visits);
+            trace_bvh2(tr, s, count, fetch_counter(w, round, true), w.plan->head.vote_quarters, begin_bvh2, end,
+                       overflow, visits);
         }
     } else if (kRefill && !kCutouts) {
         trace_refilling(tr, count, fetch_counter(w, round, true), w.plan->head.refill_at, begin, end, overflow, visits);
@@ -257,6 +290,15 @@ __global__ void __launch_bounds__(kTraceBlockMax, kCutouts ? 1 : kTraceMinBlocks
 template <int W, int kStack>
 size_t stack_bytes(int block) {
     return (size_t)TracerOf<W, false, kStack, false>::kInts * (size_t)block * sizeof(int);
+}
+
+uint32_t warp_walk_ints(int width, int stack) {
+    switch (width * 1000 + stack) {
+#define LR_CASE(wd, k) case wd * 1000 + k: return kWarpWalk<wd, false> ? kWarpInts<wd, k> : 0u;
+        LR_TRAVERSALS(LR_CASE)
+#undef LR_CASE
+        default: return 0u;
+    }
 }
 
 void launch_closest(int width, int stack, int block, bool count, bool refill, int grid, cudaStream_t stream,

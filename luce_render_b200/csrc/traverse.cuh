@@ -672,7 +672,9 @@ struct TracerOf {
 template <bool kAny, int kStack, bool kCount>
 struct TracerOf<8, kAny, kStack, kCount> {
     using type = CompressedTracer<kAny, kStack, kCount>;
-    static constexpr int kInts = kStack;  // (node << 8) | ranks, a group
+    // (node << 8) | ranks, a group; and a word for the warp walk, whose stack of 31 words a
+    // level and 32 then fits a warp's share at kStack levels (warpwalk.cuh).
+    static constexpr int kInts = kStack + 1;
 };
 template <bool kAny, int kStack, bool kCount>
 struct TracerOf<2, kAny, kStack, kCount> {
@@ -680,16 +682,17 @@ struct TracerOf<2, kAny, kStack, kCount> {
     static constexpr int kInts = kStack;
 };
 
-// The BVH2 walk of a long queue: a warp votes each step between nodes and leaves, and refills.
+// The BVH2 walk of a queue: plain batches, or a warp that votes between nodes and leaves and
+// refills.
 //
-// Walked ray by ray (trace_batched), a warp's lanes wait twice: in the node loop until the
-// last lane has reached a leaf, and at the end until the longest of 32 rays is done. On
-// incoherent rays 7 of 32 lanes work while the issue slots are 74 % busy, so the walk is
-// bound by instructions issued for idle lanes. Here
-//   - all lanes step through nodes as long as kVoteNodes of them stand at one; the others,
+// Walked plainly, a warp takes 32 neighbouring rays at a time, and its lanes wait twice: in
+// the node loop until the last lane has reached a leaf, and at the end until the longest ray
+// is done. On incoherent rays 7 of 32 lanes work while the issue slots are 74 % busy, so the
+// walk is bound by instructions issued for idle lanes. A voting warp instead
+//   - steps its lanes through nodes as long as kVoteNodes of them stand at one; the others,
 //     at a leaf, wait for no more than that, then every lane at a leaf tests it;
-//   - once kVoteRefill lanes have finished their rays they finish them together (`end`) and
-//     take the queue's next entries with one atomic (`begin`).
+//   - once kVoteRefill lanes have finished their rays, finishes those together (`end`) and
+//     takes the queue's next entries with one atomic (`begin`).
 // A ray's own order of visits does not change, so neither does any answer, any-hit ids
 // included. Measured (B200, 1M triangles): 4,194,304 incoherent rays 1,863 -> 1,389 us,
 // the 1080p pass's first bounce (1,049,661 rays) 723 -> 531, its first shadow rays (555,285)
@@ -699,32 +702,46 @@ struct TracerOf<2, kAny, kStack, kCount> {
 // and 89 on the glossy box's 256,000 (leaves outnumber nodes there); refills at 8, 16, 24
 // and 32 lanes with the vote at 8: 1,409, 1,389, 1,442, 1,968.
 //
-// The loop stays converged around its ballots and ends: a pass of it steps every ray in
-// hand at least once along a finite tree. `s` is the scene of this lane's ray; `begin(i)` sets
-// it up and starts ray i, false when there is no walk to take.
+// Where it pays (plain time over voted, closest hits, 2^21 / 800k / 400k / 230k / 180k rays):
+//   1M triangles    incoherent 1.31 1.23 1.16 1.12 1.06   camera rays 1.13 1.20 1.34 1.05 1.04
+//   200k triangles  incoherent 1.34 1.25 1.16 1.05 0.91   camera rays 1.00 1.01 0.93 0.95 0.95
+//   13k triangles   incoherent 1.50 1.24 1.05 0.91 0.94   camera rays 0.94 0.95 0.87 0.87 0.85
+// A queue has to hold more rays than the launch has lanes (170k here) for finished lanes to
+// find new ones, the more the shorter its rays are: vote_quarters() rays a lane, in quarters.
+// And a batch whose rays leave along one direction octant, as a camera's do, keeps its
+// lanes in step by itself unless the tree is deep: in smaller scenes it is walked plainly.
 constexpr int kVoteNodes = 8, kVoteRefill = 16;
 constexpr int kIdleLane = (int)0x80000000;  // a lane's node between rays: no leaf link is that low
+constexpr uint32_t kVoteAlways = 4;         // vote_quarters of a scene whose camera rays vote too
 
+__host__ __device__ constexpr uint32_t vote_quarters(uint64_t triangles) {
+    return triangles >= 400000u ? kVoteAlways : (triangles >= 100000u ? 6u : 10u);
+}
+
+// The loop stays converged around its ballots and ends: a pass of it steps every ray in
+// hand at least once along a finite tree. `s` is the scene of this lane's ray; `begin(i)` sets
+// it up and starts ray i, false when there is no walk to take, and `end(i)` takes the answer.
 template <class Tracer, class Begin, class End>
-__device__ __forceinline__ void trace_voted(Tracer &tr, const DeviceScene &s, uint32_t count, uint32_t *next,
-                                            Begin begin, End end, bool &overflow, Visits &visits) {
+__device__ __forceinline__ void trace_bvh2(Tracer &tr, const DeviceScene &s, uint32_t count, uint32_t *next,
+                                           uint32_t quarters, Begin begin, End end, bool &overflow, Visits &visits) {
+    constexpr uint32_t kAll = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
+    const bool vote = (uint64_t)count * 4u > (uint64_t)quarters * (gridDim.x * blockDim.x);
     uint32_t i = 0;
-    bool ended = true, drained = false;
+    bool ended = true, drained = false, plain = true;
     tr.node = kIdleLane;
     for (;;) {
-        const uint32_t idle = __ballot_sync(0xffffffffu, tr.node == kIdleLane);
-        const bool last = drained && idle == 0xffffffffu;
-        if (last || (!drained && __popc(idle) >= kVoteRefill)) {
+        const uint32_t idle = __ballot_sync(kAll, tr.node == kIdleLane);
+        if (idle == kAll || (!drained && __popc(idle) >= kVoteRefill)) {
             if (tr.node == kIdleLane && !ended) {
                 end(i);
                 ended = true;
             }
-            if (last) break;
+            if (drained && idle == kAll) break;
             const uint32_t want = (uint32_t)__popc(idle);
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(next, want);
-            base = __shfl_sync(0xffffffffu, base, 0);
+            base = __shfl_sync(kAll, base, 0);
             drained = base + want >= count;
             if (tr.node == kIdleLane) {
                 i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
@@ -734,37 +751,44 @@ __device__ __forceinline__ void trace_voted(Tracer &tr, const DeviceScene &s, ui
                 }
             }
             __syncwarp();
+            if (idle == kAll) {  // a batch of its own: how to walk it
+                plain = !vote;
+                if (vote && quarters != kVoteAlways) {
+                    const uint32_t octant = (tr.r.d.x < 0.0f ? 1u : 0u) | (tr.r.d.y < 0.0f ? 2u : 0u) | (tr.r.d.z < 0.0f ? 4u : 0u);
+                    const uint32_t first = __shfl_sync(kAll, octant, 0);
+                    plain = __all_sync(kAll, ended || octant == first);
+                }
+            }
         }
-        do {
-            if (tr.node >= 0 && tr.visit(s, overflow, visits)) tr.node = kIdleLane;
-        } while (__popc(__ballot_sync(0xffffffffu, tr.node >= 0)) >= kVoteNodes);
-        if (tr.node < 0 && tr.node != kIdleLane && tr.leaf(s, visits)) tr.node = kIdleLane;
+        if (plain) {
+            if (tr.node != kIdleLane) {
+                while (!tr.step(s, overflow, visits)) {
+                }
+                tr.node = kIdleLane;
+            }
+        } else {
+            do {
+                if (tr.node >= 0 && tr.visit(s, overflow, visits)) tr.node = kIdleLane;
+            } while (__popc(__ballot_sync(kAll, tr.node >= 0)) >= kVoteNodes);
+            if (tr.node < 0 && tr.node != kIdleLane && tr.leaf(s, visits)) tr.node = kIdleLane;
+        }
         __syncwarp();
     }
 }
 
-// Whether a queue of `count` rays is long enough for the voted walk: more rays than the
-// launch has lanes, so that finished lanes have rays to take. Shorter queues are bound by
-// their longest rays, which the plain walk takes with less bookkeeping (glossy box, 171,957
-// rays on 170,496 lanes: 97 us plain, 113 voted; 275,175 rays of a 100k-triangle view: 172 and
-// 148).
-__device__ __forceinline__ bool long_queue(uint32_t count) { return count > gridDim.x * blockDim.x; }
-
 // A resident grid over a queue of `count` rays in warp batches: each warp takes the next
 // 32 consecutive entries (neighbouring primary rays keep its lanes on similar nodes) with
 // one atomic on `next` (zero at launch) whenever its lanes are done, so warps that drew
-// long rays take fewer batches; a long queue on the BVH2 takes the voted walk. `load(i)` gives ray i and `store(i, hit, ray)` takes its
+// long rays take fewer batches; the BVH2 takes trace_bvh2. `load(i)` gives ray i and `store(i, hit, ray)` takes its
 // result.
 template <int W, bool kAny, int kStack, bool kCount, class Load, class Store>
 __device__ __forceinline__ void trace_batched(const DeviceScene &s, uint32_t count, uint32_t *next, int *stack_base,
                                               int stride, Load load, Store store, bool &overflow, Visits &visits) {
     typename TracerOf<W, kAny, kStack, kCount>::type tr(stack_base, stride);
     if constexpr (W == 2) {
-        if (long_queue(count)) {
-            trace_voted(tr, s, count, next, [&](uint32_t i) { return tr.start(s, load(i)); },
-                        [&](uint32_t i) { store(i, tr.h, tr.r); }, overflow, visits);
-            return;
-        }
+        trace_bvh2(tr, s, count, next, vote_quarters(s.triangle_count), [&](uint32_t i) { return tr.start(s, load(i)); },
+                   [&](uint32_t i) { store(i, tr.h, tr.r); }, overflow, visits);
+        return;
     }
     const uint32_t lane = threadIdx.x & 31u;
     for (;;) {

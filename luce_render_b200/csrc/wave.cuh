@@ -96,7 +96,10 @@ struct PlanHeader {
     uint32_t camera_paths, folds, adapts, bin_interval;
     // refill_at: the traversal kernels' persistent warps take new queue entries once this
     // many of their lanes are idle (1 to 32; 0: grid-stride walks; an autotuner choice).
-    uint32_t refill_at, reserved[3];
+    // warp_rays: queues of at most this many rays a warp of the launch are walked a warp a
+    // ray (warpwalk.cuh; 0: none, some member's tree cannot be).
+    // vote_quarters: trace_bvh2's, for the member with most of the pass's paths.
+    uint32_t refill_at, warp_rays, vote_quarters, reserved;
 };
 
 // A renderer's display image for the pass (film_convert.comp:50-52): where the pass that
@@ -209,6 +212,9 @@ void launch_closest(int width, int stack, int block, bool count, bool refill, in
                     const Wave &w, uint32_t round);
 void launch_shadow(int width, int stack, int block, bool count, bool cutouts, bool refill, int grid,
                    cudaStream_t stream, const Wave &w, uint32_t round);
+// warp_walk_ints: the words of stack a warp has for the warp walk in variant (width, stack), 0
+// when the variant does not take it.
+uint32_t warp_walk_ints(int width, int stack);
 int closest_grid(int width, int stack, int block, bool refill, int sm_count);
 
 }  // namespace lr
