@@ -310,7 +310,8 @@ int lr_launch_overhead(lr_context *ctx, uint32_t count, int32_t graph, double ou
  * free and out[1] total bytes (cudaMemGetInfo), out[2] the bytes the device's default
  * stream-ordered pool has handed out now, out[3] the most it has handed out at once since
  * the last reset; `reset_high` nonzero resets that high-water mark to the current use
- * first. lr_probe, lr_trace_rays and batch members allocate from that pool. */
+ * first. Batch members and queries of more than 8 MiB (lr_probe: 8 bytes a pixel, lr_trace_rays:
+ * 48 a ray) allocate from that pool; smaller queries stage in memory their context keeps. */
 int lr_context_memory(lr_context *ctx, int32_t reset_high, uint64_t out[4]);
 
 /* Ray queries, the ray-list form of the probe. A ray is 8 floats (origin xyz, tmin,

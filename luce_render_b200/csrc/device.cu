@@ -35,14 +35,9 @@ __device__ __forceinline__ void note_overflow(int *status, bool overflow) {
     if (overflow) atomicAdd(status, 1);
 }
 
-// probe.comp:21-34: one pixel-centre ray per pixel, row-major from the top.
-template <bool kRef, int kStack>
-__global__ void __launch_bounds__(kBlock) probe_kernel(DeviceScene s, ProbeFrame f, uint32_t *faces, float *ts,
-                                                      int *status) {
-    __shared__ int stack[kStack * kBlock];
-    const uint32_t width = (uint32_t)f.b[11], height = (uint32_t)f.b[15];
-    const uint64_t pixel = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
-    if (pixel >= (uint64_t)width * height) return;
+// probe.comp:21-34: the pixel-centre ray of pixel `pixel`, row-major from the top.
+__device__ __forceinline__ Ray probe_ray(const ProbeFrame &f, uint64_t pixel) {
+    const uint32_t width = (uint32_t)f.b[11];
     const uint32_t x = (uint32_t)(pixel % width), y = (uint32_t)(pixel / width);
     const float fx = fadd_((float)x, 0.5f), fy = fadd_((float)y, 0.5f);
     float film[3], o[3], d[3];
@@ -56,12 +51,40 @@ __global__ void __launch_bounds__(kBlock) probe_kernel(DeviceScene s, ProbeFrame
         o[k] = ortho ? fadd_(f.b[k], film[k]) : f.b[k];
         d[k] = ortho ? __fdiv_rn(fw[k], fl) : film[k];
     }
-    Ray r{make_float3(o[0], o[1], o[2]), 0.0f, make_float3(d[0], d[1], d[2]), kNoHitT};
+    return Ray{make_float3(o[0], o[1], o[2]), 0.0f, make_float3(d[0], d[1], d[2]), kNoHitT};
+}
+
+__device__ __forceinline__ uint64_t probe_pixels(const ProbeFrame &f) {
+    return (uint64_t)(uint32_t)f.b[11] * (uint32_t)f.b[15];
+}
+
+// A thread a pixel.
+template <bool kRef, int kStack>
+__global__ void __launch_bounds__(kBlock) probe_kernel(DeviceScene s, ProbeFrame f, uint32_t *faces, float *ts,
+                                                      int *status) {
+    __shared__ int stack[kStack * kBlock];
+    const uint64_t pixel = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
+    if (pixel >= probe_pixels(f)) return;
+    const Ray r = probe_ray(f, pixel);
     bool overflow = false;
     Visits visits;
     Hit h = kRef ? trace_reference<false, kStack>(s, r, stack + threadIdx.x, kBlock, overflow, visits)
                  : trace_exact<false, kStack>(s, r, stack + threadIdx.x, kBlock, overflow, visits);
     note_overflow(status, overflow);
+    faces[pixel] = h.slot >= 0 ? __ldg(&s.faces[h.slot]) : 0xffffffffu;
+    ts[pixel] = h.t;
+}
+
+// A warp a pixel, for small frames (warpwalk.cuh): their launch has a block for every four.
+__global__ void __launch_bounds__(kBlock) probe_warps_kernel(DeviceScene s, ProbeFrame f, uint32_t *faces, float *ts,
+                                                            int *status) {
+    __shared__ int stack[kBlock / 32][kWarpQueryInts];
+    const uint64_t pixel = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+    if (pixel >= probe_pixels(f)) return;
+    bool overflow = false;
+    const Hit h = walk_warp<false>(s, probe_ray(f, pixel), stack[threadIdx.x >> 5], kWarpQueryInts, overflow);
+    note_overflow(status, overflow);
+    if ((threadIdx.x & 31u) != 0u) return;
     faces[pixel] = h.slot >= 0 ? __ldg(&s.faces[h.slot]) : 0xffffffffu;
     ts[pixel] = h.t;
 }
@@ -254,6 +277,13 @@ void dispatch_reference(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, 
 template <bool kRef>
 void dispatch_probe(const lr_gpu_scene *gs, const ProbeFrame &f, uint64_t count, uint32_t *faces, float *ts,
                     int *status, cudaStream_t stream) {
+    // Up to two pixels a warp that fits the GPU: a camera's neighbouring rays keep a plain
+    // warp's lanes in step, so the warp walk pays only while the frame cannot fill the GPU.
+    constexpr uint64_t kWarps = kBlock / 32;
+    if (!kRef && count <= 2 * kWarps * warps_resident() && warp_walkable(gs->scene, kWarpQueryInts)) {
+        probe_warps_kernel<<<(unsigned)((count + kWarps - 1) / kWarps), kBlock, 0, stream>>>(gs->scene, f, faces, ts, status);
+        return;
+    }
     switch (stack_for(gs->scene.depth)) {
         case 32: launch_probe<kRef, 32>(gs, f, count, faces, ts, status, stream); break;
         case 64: launch_probe<kRef, 64>(gs, f, count, faces, ts, status, stream); break;
@@ -359,9 +389,9 @@ using namespace lr;
 
 namespace lr {
 void check_status(lr_context *ctx) {
-    int words[2] = {0, 0};
-    LR_CUDA(cudaMemcpyAsync(words, ctx->status, sizeof words, cudaMemcpyDeviceToHost, ctx->stream));
+    LR_CUDA(cudaMemcpyAsync(ctx->words, ctx->status, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     LR_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int words[2] = {ctx->words[0], ctx->words[1]};
     if (words[0] || words[1]) {
         LR_CUDA(cudaMemsetAsync(ctx->status, 0, sizeof words, ctx->stream));
         LR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -369,6 +399,45 @@ void check_status(lr_context *ctx) {
         fail(LR_TIMEOUT, "a device-side bounded wait gave up " + std::to_string(words[1]) + " times");
     }
 }
+
+namespace {
+
+// The most a context keeps for staging small queries: a million-pixel probe, 174k rays. The
+// stream-ordered pool gives freed memory back to the device at every wait, so a small query
+// that allocates from it pays for mapping memory each time: a one-pixel probe took 480 us,
+// 4,099 host rays 600, most of it that (26 and 62 us through the staging; a 640x359 probe
+// 800 -> 334). Larger queries still allocate, and copy far longer.
+constexpr size_t kPadMost = 8u << 20;
+
+// Makes the context's staging hold `bytes`; false when that is more than it keeps.
+bool pad_holds(lr_context *ctx, uint64_t bytes) {
+    if (bytes > kPadMost) return false;
+    if (bytes <= ctx->pad_bytes) return true;
+    size_t size = 64u << 10;
+    while (size < bytes) size <<= 1;
+    if (ctx->pad) LR_CUDA(cudaFree(ctx->pad));
+    ctx->pad = nullptr;
+    ctx->pad_bytes = 0;
+    if (ctx->pad_host) LR_CUDA(cudaFreeHost(ctx->pad_host));
+    ctx->pad_host = nullptr;
+    LR_CUDA(cudaMalloc(&ctx->pad, size));
+    LR_CUDA(cudaMallocHost(&ctx->pad_host, size));
+    ctx->pad_bytes = size;
+    return true;
+}
+
+// Runs a query's queueing and waiting; whatever was queued has finished when it fails.
+template <class F>
+void staged(lr_context *ctx, F &&body) {
+    try {
+        body();
+    } catch (...) {
+        cudaStreamSynchronize(ctx->stream);
+        throw;
+    }
+}
+
+}  // namespace
 }  // namespace lr
 
 extern "C" {
@@ -398,6 +467,7 @@ int lr_context_create_ex(int device, int priority, lr_context **out) {
         // Status words at byte 0, traversal counts at byte 16, the ray queries' batch
         // cursor at byte 32 (kBatchCursor ints in).
         LR_CUDA(cudaMalloc(&ctx->status, 64));
+        LR_CUDA(cudaMallocHost(&ctx->words, 64));
         LR_CUDA(cudaMemsetAsync(ctx->status, 0, 64, ctx->stream));
         ctx->counts = (unsigned long long *)((char *)ctx->status + 16);
         LR_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -410,6 +480,9 @@ void lr_context_destroy(lr_context *ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->status) cudaFree(ctx->status);
+    if (ctx->words) cudaFreeHost(ctx->words);
+    if (ctx->pad) cudaFree(ctx->pad);
+    if (ctx->pad_host) cudaFreeHost(ctx->pad_host);
     if (ctx->start) cudaEventDestroy(ctx->start);
     if (ctx->stop) cudaEventDestroy(ctx->stop);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -419,7 +492,6 @@ void lr_context_destroy(lr_context *ctx) {
 int lr_context_synchronize(lr_context *ctx) {
     return guarded([&] {
         if (!ctx) fail(LR_INVALID, "no context");
-        LR_CUDA(cudaStreamSynchronize(ctx->stream));
         check_status(ctx);
     });
 }
@@ -679,6 +751,22 @@ int lr_probe(lr_context *ctx, const lr_gpu_scene *gs, const lr_frame *frame, uin
         ProbeFrame f;
         pack_frame(*frame, f.b);
         LR_CUDA(cudaSetDevice(ctx->device));
+        if (pad_holds(ctx, count * 8)) {
+            staged(ctx, [&] {
+                uint32_t *d_faces = (uint32_t *)ctx->pad;
+                float *d_ts = (float *)(ctx->pad + count * 4);
+                if (flags & LR_TRACE_REFERENCE)
+                    dispatch_probe<true>(gs, f, count, d_faces, d_ts, ctx->status, ctx->stream);
+                else
+                    dispatch_probe<false>(gs, f, count, d_faces, d_ts, ctx->status, ctx->stream);
+                LR_CUDA(cudaGetLastError());
+                LR_CUDA(cudaMemcpyAsync(ctx->pad_host, ctx->pad, count * 8, cudaMemcpyDeviceToHost, ctx->stream));
+                check_status(ctx);
+            });
+            std::memcpy(faces, ctx->pad_host, count * 4);
+            std::memcpy(distances, ctx->pad_host + count * 4, count * 4);
+            return;
+        }
         void *buffer = nullptr;
         LR_CUDA(cudaMallocAsync(&buffer, count * 8, ctx->stream));
         uint32_t *d_faces = (uint32_t *)buffer;
@@ -691,7 +779,6 @@ int lr_probe(lr_context *ctx, const lr_gpu_scene *gs, const lr_frame *frame, uin
         LR_CUDA(cudaMemcpyAsync(faces, d_faces, count * 4, cudaMemcpyDeviceToHost, ctx->stream));
         LR_CUDA(cudaMemcpyAsync(distances, d_ts, count * 4, cudaMemcpyDeviceToHost, ctx->stream));
         LR_CUDA(cudaFreeAsync(buffer, ctx->stream));
-        LR_CUDA(cudaStreamSynchronize(ctx->stream));
         check_status(ctx);
     });
 }
@@ -768,13 +855,12 @@ int lr_probe_static(lr_context *ctx, const lr_gpu_scene *gs, const lr_frame *fra
             LR_CUDA(cudaGetLastError());
             LR_CUDA(cudaMemcpyAsync(faces, d_faces, count * 4, cudaMemcpyDeviceToHost, ctx->stream));
             LR_CUDA(cudaMemcpyAsync(distances, d_ts, count * 4, cudaMemcpyDeviceToHost, ctx->stream));
-            LR_CUDA(cudaStreamSynchronize(ctx->stream));
+            check_status(ctx);
         } catch (...) {
             // Whatever was queued finishes before the array is handed to the next call.
             cudaStreamSynchronize(ctx->stream);
             throw;
         }
-        check_status(ctx);
     });
 }
 
@@ -846,6 +932,18 @@ int lr_trace_rays(lr_context *ctx, const lr_gpu_scene *gs, const float *rays, ui
         if (!ctx || !gs || (count && (!rays || !hits))) fail(LR_INVALID, "a ray query needs rays and room for hits");
         if (count == 0) return;
         LR_CUDA(cudaSetDevice(ctx->device));
+        if (count <= kPadMost / 48 && pad_holds(ctx, count * 48)) {
+            char *d_hits = ctx->pad + count * 32;
+            std::memcpy(ctx->pad_host, rays, count * 32);
+            staged(ctx, [&] {
+                LR_CUDA(cudaMemcpyAsync(ctx->pad, ctx->pad_host, count * 32, cudaMemcpyHostToDevice, ctx->stream));
+                trace_device(ctx, gs, ctx->pad, count, d_hits, flags);
+                LR_CUDA(cudaMemcpyAsync(ctx->pad_host, d_hits, count * 16, cudaMemcpyDeviceToHost, ctx->stream));
+                check_status(ctx);
+            });
+            std::memcpy(hits, ctx->pad_host, count * 16);
+            return;
+        }
         void *buffer = nullptr;
         LR_CUDA(cudaMallocAsync(&buffer, count * 48, ctx->stream));
         void *d_hits = (char *)buffer + count * 32;
@@ -853,7 +951,6 @@ int lr_trace_rays(lr_context *ctx, const lr_gpu_scene *gs, const float *rays, ui
         trace_device(ctx, gs, buffer, count, d_hits, flags);
         LR_CUDA(cudaMemcpyAsync(hits, d_hits, count * 16, cudaMemcpyDeviceToHost, ctx->stream));
         LR_CUDA(cudaFreeAsync(buffer, ctx->stream));
-        LR_CUDA(cudaStreamSynchronize(ctx->stream));
         check_status(ctx);
     });
 }

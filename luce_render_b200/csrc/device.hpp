@@ -69,10 +69,18 @@ struct lr_context {
     int *status = nullptr;
     // Traversal work of counted ray queries: interior visits, triangle tests.
     unsigned long long *counts = nullptr;
+    // Where small host-side queries stage their rays and results: device memory and page-locked
+    // host memory of `pad_bytes` each (lr::kPadMost at most), made by the first such query, grown
+    // by a larger one, freed with the context; `words` holds the status words read back. Every
+    // query has waited for its work when it returns, and one thread drives a context.
+    char *pad = nullptr, *pad_host = nullptr;
+    size_t pad_bytes = 0;
+    int *words = nullptr;
 };
 
 namespace lr {
-// Reads and clears the context's status words; fails when one is set.
+// Waits for the context's stream, then reads and clears its status words; fails when one is
+// set.
 void check_status(lr_context *ctx);
 // lr_probe_static's set-up on `device` (the device address of its static array, looked up
 // once per device, which may load the module there); returns the address.
