@@ -13,7 +13,7 @@
 //      thread waiting on another;
 //   3. the watertight path's widened boxes from the exact ones, with the widening taken
 //      again from the new root box (2^-16 of the scene's scale, one more float step);
-//   4. the 4-wide collapse's child boxes, copied from the BVH2 slots they came from, the
+//   4. (in the same launch) the 4-wide collapse's child boxes, copied from the BVH2 slots they came from, the
 //      compressed 8-wide nodes quantized again from those boxes (quantize.hpp), and the
 //      8-wide tree's plain boxes (DeviceWide::boxes).
 // With the points unchanged a refit leaves every array bit for bit as the upload made it,
@@ -181,94 +181,150 @@ __global__ void leaf_root_kernel(const float *positions, const uint32_t *indices
     }
 }
 
-// Step 3: the float4s 0..2 of every entry hold (lo, hi, lo, hi) pairs.
-__global__ void widen_kernel(uint64_t count, const float4 *exact, float4 *widened, float delta) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t e = i / 3, k = i % 3;
-        const float4 v = exact[e * 4 + k];
+// The widening of a root box (device.cu's build_layout, the same doubles): 2^-16 of the scene's
+// scale, its largest magnitude or extent and at least 1.
+__host__ __device__ inline float widening(const float *root) {
+    double scale = 1.0;
+    for (int k = 0; k < 3; k++) {
+        const double lo = fabs((double)root[k]), hi = fabs((double)root[4 + k]), extent = (double)(root[4 + k] - root[k]);
+        scale = scale < lo ? lo : scale;
+        scale = scale < hi ? hi : scale;
+        scale = scale < extent ? extent : scale;
+    }
+    return (float)(scale * (1.0 / 65536.0));
+}
+
+// The box a wide child slot was collapsed from: a BVH2 slot's or the root's.
+__device__ __forceinline__ Box source_box(uint32_t source, const float4 *exact, const float *root_box) {
+    if (source != kRefitRoot) return read_side(exact, source >> 1, source & 1u);
+    Box b;
+    for (int k = 0; k < 3; k++) {
+        b.lo[k] = __ldcg(&root_box[k]);
+        b.hi[k] = __ldcg(&root_box[4 + k]);
+    }
+    return b;
+}
+
+// One child slot of the 8-wide tree, by the lane of its slot among a node's eight: its plain
+// box (DeviceWide::boxes) and its bytes of the compressed node, quantized together with the
+// node's other lanes exactly as quantize_node (quantize.hpp) does alone -- the origin and
+// extent by a minimum and a maximum over the lanes, an axis' exponent raised until every lane's
+// planes fit. A thread a node took 111 us on 64,673 nodes (each a loop over 8 x 3 planes, half a
+// wave of threads), half of the refit. Every lane of the warp calls it; `slot` past the end of the tree has none of a node's.
+__device__ __forceinline__ void wide8_slot(uint64_t slot, bool valid, const uint32_t *sources, const float4 *exact,
+                                           const float *root_box, float delta, float4 *nodes, float4 *boxes) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, c = (uint32_t)slot & 7u, first = lane & 24u;
+    const uint32_t source = valid ? __ldg(&sources[slot]) : 0xffffffffu;
+    const bool taken = source != 0xffffffffu;
+    float *node = reinterpret_cast<float *>(nodes + (slot >> 3) * kQNodeFloat4s);
+    Box b{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+    if (taken) {
+        b = source_box(source, exact, root_box);
+        for (int k = 0; k < 3; k++) {
+            b.lo[k] = widen_lo(b.lo[k], delta);
+            b.hi[k] = widen_hi(b.hi[k], delta);
+        }
+        lo = make_float4(b.lo[0], b.lo[1], b.lo[2], node[4 + c]);
+        hi = make_float4(b.hi[0], b.hi[1], b.hi[2], 1.0f);
+    }
+    if (valid) {
+        boxes[2 * slot] = lo;
+        boxes[2 * slot + 1] = hi;
+    }
+    const uint32_t occupied = (__ballot_sync(kAll, taken) >> first) & 0xffu;
+    float origin[3];
+    uint32_t exps = 0;
+    uint8_t *bytes = reinterpret_cast<uint8_t *>(node + 12);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        float low = b.lo[k], top = b.hi[k];
+#pragma unroll
+        for (int step = 4; step > 0; step >>= 1) {
+            low = fminf(low, __shfl_xor_sync(kAll, low, step));
+            top = fmaxf(top, __shfl_xor_sync(kAll, top, step));
+        }
+        origin[k] = low;
+        uint32_t e = occupied ? q_exponent(top - low) : 254u;
+        int32_t ql = 255, qh = 0;
+        for (;;) {
+            bool fits = true;
+            if (taken) {
+                const float s = q_step(e);
+                ql = (int32_t)q_floor((b.lo[k] - low) / s);
+                if (ql < 0) ql = 0;
+                while (ql > 0 && low + (float)ql * s > b.lo[k]) ql--;
+                qh = (int32_t)q_floor((b.hi[k] - low) / s);
+                if (qh < 0) qh = 0;
+                while (qh < 256 && low + (float)qh * s < b.hi[k]) qh++;
+                fits = qh <= 255 && low + (float)ql * s <= b.lo[k];
+            }
+            const bool done = ((__ballot_sync(kAll, fits) >> first) & 0xffu) == 0xffu || e >= 254u;
+            if (__all_sync(kAll, done)) break;
+            if (!done) e++;
+        }
+        exps |= e << (8 * k);
+        if (valid) {
+            bytes[16 * k + c] = (uint8_t)ql;
+            bytes[16 * k + 8 + c] = (uint8_t)qh;
+        }
+    }
+    if (valid && c == 0u)
+        *reinterpret_cast<float4 *>(node) =
+            make_float4(origin[0], origin[1], origin[2], __uint_as_float(exps | occupied << 24));
+}
+
+// Steps 3 and 4 in one launch, after the climb: the widened BVH2 boxes, the 4-wide tree's and
+// the 8-wide tree's. The widening comes from the new root box on the device, worked out once a
+// block, so nothing waits for the host between the climb and here (which took a copy, a wait and
+// a launch). On 1,048,576 triangles 30 us, latency of the wide slots' scattered box reads for the
+// most part, against 8 + 10 + 111 + 9 in launches of their own; the refit and a query of 32,768
+// rays 314 -> 201 us. The climb is what is left (63 us).
+__global__ void __launch_bounds__(256) boxes_kernel(uint64_t entries, float4 *widened, uint64_t slots4, const uint32_t *sources4,
+                                                    float4 *nodes4, uint64_t slots8, const uint32_t *sources8,
+                                                    float4 *nodes8, float4 *boxes8, const float4 *exact,
+                                                    const float *root_box) {
+    __shared__ float block_delta;
+    if (threadIdx.x == 0) {
+        float root[8];
+        for (int k = 0; k < 8; k++) root[k] = __ldcg(&root_box[k]);
+        block_delta = widening(root);
+    }
+    __syncthreads();
+    const float delta = block_delta;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, at = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    // The 8-wide tree first: its lanes work longest. Whole warps, so that a node's lanes stay together.
+    for (uint64_t i = at; i < ((slots8 + 31) & ~(uint64_t)31); i += stride)
+        wide8_slot(i, i < slots8, sources8, exact, root_box, delta, nodes8, boxes8);
+    // The 4-wide tree's child slot i; empty slots keep their inverted boxes.
+    for (uint64_t i = at; i < slots4; i += stride) {
+        const uint32_t source = __ldg(&sources4[i]);
+        if (source == 0xffffffffu) continue;
+        const Box b = source_box(source, exact, root_box);
+        float *base = reinterpret_cast<float *>(nodes4 + (i >> 2) * 7) + (i & 3);
+        for (int k = 0; k < 3; k++) {
+            base[8 * k] = widen_lo(b.lo[k], delta);
+            base[8 * k + 4] = widen_hi(b.hi[k], delta);
+        }
+    }
+    // The float4s 0..2 of every BVH2 entry hold (lo, hi, lo, hi) pairs.
+    for (uint64_t i = at; i < entries * 3; i += stride) {
+        const uint64_t e = i / 3, k = i - e * 3;
+        const float4 v = __ldcg(&exact[e * 4 + k]);
         widened[e * 4 + k] = make_float4(widen_lo(v.x, delta), widen_hi(v.y, delta), widen_lo(v.z, delta),
                                          widen_hi(v.w, delta));
     }
 }
 
-// Step 4: 4-wide node n's child slot i from the BVH2 slot (or the root) it was collapsed
-// from; empty slots keep their inverted boxes.
-__global__ void wide_kernel(uint64_t slots, int width, const uint32_t *sources, const float4 *exact,
-                            const float *root_box, float delta, float4 *nodes) {
-    const int per_node = 7, planes = width / 4;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < slots; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t source = sources[i];
-        if (source == 0xffffffffu) continue;
-        Box b;
-        if (source == kRefitRoot) {
-            for (int k = 0; k < 3; k++) {
-                b.lo[k] = root_box[k];
-                b.hi[k] = root_box[4 + k];
-            }
-        } else {
-            b = read_side(exact, source >> 1, source & 1u);
-        }
-        const uint64_t n = i / width;
-        const int slot = (int)(i % width);
-        float *base = reinterpret_cast<float *>(nodes + n * per_node);
-        for (int k = 0; k < 3; k++) {
-            base[((2 * k) * planes) * 4 + slot] = widen_lo(b.lo[k], delta);
-            base[((2 * k + 1) * planes) * 4 + slot] = widen_hi(b.hi[k], delta);
-        }
-    }
-}
-
-// Step 4 for the compressed 8-wide tree: node n quantized again (quantize.hpp) from its
-// children's BVH2 boxes (or the root's), widened as at upload; its links and occupied
-// slots stay.
-__global__ void quantize_kernel(uint64_t count, const uint32_t *sources, const float4 *exact, const float *root_box,
-                                float delta, float4 *nodes) {
-    for (uint64_t n = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; n < count; n += (uint64_t)gridDim.x * blockDim.x) {
-        float *node = reinterpret_cast<float *>(nodes + n * kQNodeFloat4s);
-        const uint32_t occupied = __float_as_uint(node[3]) >> 24;
-        float lo[8][3], hi[8][3];
-        int links[8];
-        for (int c = 0; c < 8; c++) {
-            links[c] = __float_as_int(node[4 + c]);
-            if (!((occupied >> c) & 1u)) continue;
-            const uint32_t source = sources[n * 8 + c];
-            Box b;
-            if (source == kRefitRoot) {
-                for (int k = 0; k < 3; k++) {
-                    b.lo[k] = root_box[k];
-                    b.hi[k] = root_box[4 + k];
-                }
-            } else {
-                b = read_side(exact, source >> 1, source & 1u);
-            }
-            for (int k = 0; k < 3; k++) {
-                lo[c][k] = widen_lo(b.lo[k], delta);
-                hi[c][k] = widen_hi(b.hi[k], delta);
-            }
-        }
-        float out[kQNodeFloat4s * 4];
-        quantize_node(occupied, lo, hi, links, out);
-        for (int k = 0; k < kQNodeFloat4s * 4; k++) node[k] = out[k];
-    }
-}
-
-// DeviceWide::boxes: a thread a child slot, its box from the BVH2 slot (or the root) it was
-// collapsed from, its link from the compressed node.
+// The plain boxes alone, for an upload (its other boxes come from the host).
 __global__ void wide_boxes_kernel(uint64_t slots, const uint32_t *sources, const float4 *exact, const float *root_box,
                                   float delta, const float4 *nodes, float4 *boxes) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < slots; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t source = __ldg(&sources[i]);
         float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
         if (source != 0xffffffffu) {
-            Box b;
-            if (source == kRefitRoot) {
-                for (int k = 0; k < 3; k++) {
-                    b.lo[k] = root_box[k];
-                    b.hi[k] = root_box[4 + k];
-                }
-            } else {
-                b = read_side(exact, source >> 1, source & 1u);
-            }
+            const Box b = source_box(source, exact, root_box);
             const float link = __ldg(reinterpret_cast<const float *>(nodes + (i >> 3) * kQNodeFloat4s + 1) + (i & 7u));
             lo = make_float4(widen_lo(b.lo[0], delta), widen_lo(b.lo[1], delta), widen_lo(b.lo[2], delta), link);
             hi = make_float4(widen_hi(b.hi[0], delta), widen_hi(b.hi[1], delta), widen_hi(b.hi[2], delta), 1.0f);
@@ -331,33 +387,22 @@ void refit_scene(lr_gpu_scene *gs, cudaStream_t stream) {
         leaf_root_kernel<<<1, 32, 0, stream>>>(s.positions, s.indices, s.bvh.root, gs->root_box);
     }
     LR_CUDA(cudaGetLastError());
+    const uint64_t slots4 = s.wide4.width ? gs->wide4_nodes * 4 : 0, slots8 = s.wide8.width ? gs->wide8_nodes * 8 : 0;
+    if (E > 0 || slots4 || slots8)
+        boxes_kernel<<<grid_for(std::max(E * 3, slots8), sms), 256, 0, stream>>>(
+            E, widened, slots4, gs->wide4_sources, const_cast<float4 *>(s.wide4.nodes), slots8, gs->wide8_sources,
+            const_cast<float4 *>(s.wide8.nodes), const_cast<float4 *>(s.wide8.boxes), exact, gs->root_box);
+    LR_CUDA(cudaGetLastError());
     float root[8];
     LR_CUDA(cudaMemcpyAsync(root, gs->root_box, sizeof root, cudaMemcpyDeviceToHost, stream));
     LR_CUDA(cudaStreamSynchronize(stream));
-    // The widening as the upload takes it (device.cu's build_layout), from the new root box.
-    double scale = 1.0;
-    for (int k = 0; k < 3; k++) {
-        scale = std::max(scale, (double)std::fabs(root[k]));
-        scale = std::max(scale, (double)std::fabs(root[4 + k]));
-        scale = std::max(scale, (double)(root[4 + k] - root[k]));
-    }
-    const float delta = (float)std::ldexp(scale, -16);
+    const float delta = widening(root);
     for (int k = 0; k < 3; k++) {
         s.ref_bvh.root_lo[k] = root[k];
         s.ref_bvh.root_hi[k] = root[4 + k];
         s.bvh.root_lo[k] = host_widen_down(root[k], delta);
         s.bvh.root_hi[k] = host_widen_up(root[4 + k], delta);
     }
-    if (E > 0) widen_kernel<<<grid_for(E * 3, sms), 256, 0, stream>>>(E * 3, exact, widened, delta);
-    if (s.wide4.width)
-        wide_kernel<<<grid_for(gs->wide4_nodes * 4, sms), 256, 0, stream>>>(
-            gs->wide4_nodes * 4, 4, gs->wide4_sources, exact, gs->root_box, delta, const_cast<float4 *>(s.wide4.nodes));
-    if (s.wide8.width)
-        quantize_kernel<<<grid_for(gs->wide8_nodes, sms), 256, 0, stream>>>(
-            gs->wide8_nodes, gs->wide8_sources, exact, gs->root_box, delta, const_cast<float4 *>(s.wide8.nodes));
-    fill_wide_boxes(gs, delta, stream);
-    LR_CUDA(cudaGetLastError());
-    LR_CUDA(cudaStreamSynchronize(stream));
     gs->refits++;
 }
 
