@@ -220,12 +220,12 @@ unsigned warps_resident() {
     return (unsigned)resident;
 }
 
-// Short closest-hit queries of the default width a warp a ray: at most kWarpRays rays a
+// Short closest-hit queries of the default width a warp a ray: at most warp_rays_for rays a
 // resident warp, on a scene whose 8-wide tree fits the stack.
 bool launch_warps(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, float4 *hits, int *status, cudaStream_t stream) {
     constexpr uint64_t kWarps = kBlock / 32;
     const unsigned resident = warps_resident();
-    if (n > kWarpRays * kWarps * (uint64_t)resident || !warp_walkable(gs->scene, kWarpQueryInts)) return false;
+    if (n > warp_rays_for(gs->scene.triangle_count) * kWarps * (uint64_t)resident || !warp_walkable(gs->scene, kWarpQueryInts)) return false;
     uint32_t *next = (uint32_t *)(status + kBatchCursor);
     LR_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
     const unsigned grid = (unsigned)std::min<uint64_t>((n + kWarps - 1) / kWarps, resident);

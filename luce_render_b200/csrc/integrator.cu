@@ -1676,7 +1676,7 @@ bool launch_pass(WaveHost *h, bool dry = false, int only = -1) {
                         (cutouts ? kCutoutVariant : 0) + block_index * kBlockVariant +
                         (h->refill_at ? kRefillVariant : 0) + thin * kThinVariant;
     staging->head = PlanHeader{n, used, converts, dry ? 1u : 0u, camera_paths, folds, adapts, h->bin_interval,
-                               h->refill_at, walkable ? kWarpRays : 0u, vote_quarters(most_triangles), 0u};
+                               h->refill_at, walkable ? warp_rays_for(most_triangles) : 0u, vote_quarters(most_triangles), 0u};
     staging->display = PlanDisplay{0ull, h->display_scale, h->display_view, 0u, 0u};
     if (h->display_block && converts > 0) {
         rec.display_slot = free_display_slot(h);

@@ -24,11 +24,16 @@
 
 namespace lr {
 
-// Rays a warp up to which a queue takes the warp walk: measured against the BVH2 walk on
-// 4,736 warps, 3,326 rays of a 100k-triangle view 91 -> 20 us, 26,548 of a 1M-triangle one 136
-// -> 67, 30,000 incoherent ones 98 -> 56, 60,000 105 -> 95, 100,000 112 -> 146; on a 34-triangle
-// box 3,234 rays 26 -> 13, 14,009 27 -> 23, 19,807 25 -> 27, 65,536 21 -> 54.
-constexpr uint32_t kWarpRays = 8;
+// Rays a warp of the launch up to which a queue is walked a warp a ray, by the scene's
+// triangles: the shallower the tree, the shorter the chain a lane would walk. Measured against
+// the BVH2 walk on 4,736 warps: on a 34-triangle box 3,234 rays 26 -> 13 us, 14,009 27 -> 23,
+// 19,807 25 -> 27; on a 15k-triangle box 16,851 76 -> 33, 56,286 78 -> 73; on 100k triangles 3,326
+// 91 -> 20, 53,621 109 -> 100; on 1M 26,548 136 -> 67, 60,000 105 -> 95, 100,000 112 -> 146. In
+// whole passes, where a round's shadow rays share the machine, 8 beats 12 on the 15k-triangle
+// box (3,008 against 3,130 us) and 4 beats 8 on the 34-triangle one (637 against 662).
+__host__ __device__ constexpr uint32_t warp_rays_for(uint64_t triangles) {
+    return triangles < 1024u ? 4u : 8u;
+}
 
 constexpr uint32_t warp_stack_ints(uint32_t levels) { return 31u * levels + 32u; }
 
