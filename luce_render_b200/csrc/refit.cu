@@ -47,23 +47,22 @@ __device__ __forceinline__ void write_side(float4 *entries, uint32_t e, uint32_t
     __stcg(reinterpret_cast<float2 *>(&entries[(size_t)e * 4 + 2]) + side, make_float2(b.lo[2], b.hi[2]));
 }
 
-// A leaf's box from its triangles' corners: 12 bytes of indices a triangle and the points
-// (which stay in L2), not the 48-byte triangle records.
-__device__ __forceinline__ Box leaf_box(const float *positions, const uint32_t *indices, int link) {
+// A leaf's box from its triangles' records, which the launch before wrote (they are in L2): three
+// 16-byte loads a triangle, where its indices and points took twelve 4-byte ones (the climb 63 ->
+// 60 us on 1,048,576 triangles: its chain of atomics up the tree is the rest).
+__device__ __forceinline__ Box leaf_box(const float4 *tris, int link) {
     const uint32_t code = (uint32_t)(-1 - link);
     const uint32_t first = code >> kLeafShift, count = (code & ((1u << kLeafShift) - 1u)) + 1u;
     Box b{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
-    for (uint32_t t = first; t < first + count; t++)
-        for (uint32_t c = 0; c < 3; c++) {
-            const float *v = &positions[(size_t)__ldg(&indices[(size_t)t * 3 + c]) * 3];
-            const float x = __ldg(v), y = __ldg(v + 1), z = __ldg(v + 2);
-            b.lo[0] = fminf(b.lo[0], x);
-            b.lo[1] = fminf(b.lo[1], y);
-            b.lo[2] = fminf(b.lo[2], z);
-            b.hi[0] = fmaxf(b.hi[0], x);
-            b.hi[1] = fmaxf(b.hi[1], y);
-            b.hi[2] = fmaxf(b.hi[2], z);
-        }
+    for (uint32_t i = 0; i < count * 3u; i++) {
+        const float4 v = __ldg(&tris[(size_t)first * 3 + i]);
+        b.lo[0] = fminf(b.lo[0], v.x);
+        b.lo[1] = fminf(b.lo[1], v.y);
+        b.lo[2] = fminf(b.lo[2], v.z);
+        b.hi[0] = fmaxf(b.hi[0], v.x);
+        b.hi[1] = fmaxf(b.hi[1], v.y);
+        b.hi[2] = fmaxf(b.hi[2], v.z);
+    }
     return b;
 }
 
@@ -137,7 +136,7 @@ __device__ __forceinline__ uint32_t add_acq_rel(uint32_t *counter, uint32_t valu
 // Step 2. `levels` bounds a climb (the BVH2's depth + 1), so a damaged parent table can
 // only end a climb early, never loop. The next parent link is fetched before the atomic
 // (the table is read-only), so it is not on the climb's chain of dependent latencies.
-__global__ void climb_kernel(uint32_t entries, const float *positions, const uint32_t *indices, float4 *exact,
+__global__ void climb_kernel(uint32_t entries, const float4 *tris, float4 *exact,
                              const uint32_t *parents, uint32_t *counters, float *root_box, uint32_t levels) {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= entries) return;
@@ -146,7 +145,7 @@ __global__ void climb_kernel(uint32_t entries, const float *positions, const uin
     uint32_t leaves = 0;
     for (uint32_t side = 0; side < 2; side++)
         if (link[side] < 0) {
-            write_side(exact, e, side, leaf_box(positions, indices, link[side]));
+            write_side(exact, e, side, leaf_box(tris, link[side]));
             leaves++;
         }
     if (leaves == 0) return;
@@ -172,9 +171,9 @@ __global__ void climb_kernel(uint32_t entries, const float *positions, const uin
 }
 
 // A scene whose root is a leaf (at most 16 triangles): its box.
-__global__ void leaf_root_kernel(const float *positions, const uint32_t *indices, int root, float *root_box) {
+__global__ void leaf_root_kernel(const float4 *tris, int root, float *root_box) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const Box b = leaf_box(positions, indices, root);
+    const Box b = leaf_box(tris, root);
     for (int k = 0; k < 3; k++) {
         root_box[k] = b.lo[k];
         root_box[4 + k] = b.hi[k];
@@ -280,7 +279,7 @@ __device__ __forceinline__ void wide8_slot(uint64_t slot, bool valid, const uint
 // block, so nothing waits for the host between the climb and here (which took a copy, a wait and
 // a launch). On 1,048,576 triangles 30 us, latency of the wide slots' scattered box reads for the
 // most part, against 8 + 10 + 111 + 9 in launches of their own; the refit and a query of 32,768
-// rays 314 -> 201 us. The climb is what is left (63 us).
+// rays 314 -> 201 us. The climb is what is left (60 us).
 __global__ void __launch_bounds__(256) boxes_kernel(uint64_t entries, float4 *widened, uint64_t slots4, const uint32_t *sources4,
                                                     float4 *nodes4, uint64_t slots8, const uint32_t *sources8,
                                                     float4 *nodes8, float4 *boxes8, const float4 *exact,
@@ -380,11 +379,11 @@ void refit_scene(lr_gpu_scene *gs, cudaStream_t stream) {
     const uint64_t E = s.entry_count;
     if (E > 0) {
         LR_CUDA(cudaMemsetAsync(gs->counters, 0, E * sizeof(uint32_t), stream));
-        climb_kernel<<<(unsigned)((E + 127) / 128), 128, 0, stream>>>((uint32_t)E, s.positions, s.indices, exact,
+        climb_kernel<<<(unsigned)((E + 127) / 128), 128, 0, stream>>>((uint32_t)E, tris, exact,
                                                                        gs->parents, gs->counters, gs->root_box,
                                                                        s.depth + 2);
     } else {
-        leaf_root_kernel<<<1, 32, 0, stream>>>(s.positions, s.indices, s.bvh.root, gs->root_box);
+        leaf_root_kernel<<<1, 32, 0, stream>>>(tris, s.bvh.root, gs->root_box);
     }
     LR_CUDA(cudaGetLastError());
     const uint64_t slots4 = s.wide4.width ? gs->wide4_nodes * 4 : 0, slots8 = s.wide8.width ? gs->wide8_nodes * 8 : 0;
