@@ -580,7 +580,7 @@ def refit(lr, scenes, ctx, dist, repeats: int = 10) -> dict:
             "host_compile_ms": compile_s * 1e3, "host_upload_ms": upload_s * 1e3,
             "speedup_vs_host_rebuild": (compile_s + upload_s) * 1e3 / refit_ms,
             "timing": "device refit: CUDA events on the context's stream around the call (it waits for the new "
-                      "root box between launches), median of 10; host rebuild: wall clock",
+                      "root box at its end), median of 10; host rebuild: wall clock",
             "device_build": build_info}
 
 
@@ -665,7 +665,7 @@ def overhead(lr, scenes, ctx, dist) -> dict:
     r.destroy()
     sc.close()
     return {"launch_chains": chains, "empty_pass_ms": ms / 200.0,
-            "kernels_per_pass": 1 + 3 * (BOUNCES + 1) + 5,
+            "kernels_per_pass": 1 + 3 * (BOUNCES + 1) + 2,
             "timing": "chains: best of 5, CUDA events and the host clock; passes: CUDA events on the context "
                       "stream over 200 passes of 64 paths (two lanes, graphs)"}
 
@@ -914,7 +914,7 @@ def main():
                     "d2h_bytes_per_step": WIDTH * HEIGHT * 16},
             # a pass: camera; closest, shade and shadow each round; finish, fold, the two
             # adaptive phases and convert (the launch list in profiles/ counts the same)
-            "gpu_launches": K * (1 + 3 * (BOUNCES + 1) + 5),
+            "gpu_launches": K * (1 + 3 * (BOUNCES + 1) + 2),
             "clocks": clock_info,
             "light_traced": traced_info,
             "cornell": cornell_info,
