@@ -389,6 +389,7 @@ using namespace lr;
 
 namespace lr {
 void check_status(lr_context *ctx) {
+    std::lock_guard<std::recursive_mutex> turn(ctx->staging);
     LR_CUDA(cudaMemcpyAsync(ctx->words, ctx->status, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     LR_CUDA(cudaStreamSynchronize(ctx->stream));
     const int words[2] = {ctx->words[0], ctx->words[1]};
@@ -409,10 +410,9 @@ namespace {
 // 800 -> 334). Larger queries still allocate, and copy far longer.
 constexpr size_t kPadMost = 8u << 20;
 
-// Makes the context's staging hold `bytes`; false when that is more than it keeps.
-bool pad_holds(lr_context *ctx, uint64_t bytes) {
-    if (bytes > kPadMost) return false;
-    if (bytes <= ctx->pad_bytes) return true;
+// Makes the context's staging hold `bytes`, at most kPadMost.
+void pad_hold(lr_context *ctx, uint64_t bytes) {
+    if (bytes <= ctx->pad_bytes) return;
     size_t size = 64u << 10;
     while (size < bytes) size <<= 1;
     if (ctx->pad) LR_CUDA(cudaFree(ctx->pad));
@@ -423,7 +423,6 @@ bool pad_holds(lr_context *ctx, uint64_t bytes) {
     LR_CUDA(cudaMalloc(&ctx->pad, size));
     LR_CUDA(cudaMallocHost(&ctx->pad_host, size));
     ctx->pad_bytes = size;
-    return true;
 }
 
 // Runs a query's queueing and waiting; whatever was queued has finished when it fails.
@@ -751,7 +750,9 @@ int lr_probe(lr_context *ctx, const lr_gpu_scene *gs, const lr_frame *frame, uin
         ProbeFrame f;
         pack_frame(*frame, f.b);
         LR_CUDA(cudaSetDevice(ctx->device));
-        if (pad_holds(ctx, count * 8)) {
+        if (count <= kPadMost / 8) {
+            std::lock_guard<std::recursive_mutex> turn(ctx->staging);
+            pad_hold(ctx, count * 8);
             staged(ctx, [&] {
                 uint32_t *d_faces = (uint32_t *)ctx->pad;
                 float *d_ts = (float *)(ctx->pad + count * 4);
@@ -932,7 +933,9 @@ int lr_trace_rays(lr_context *ctx, const lr_gpu_scene *gs, const float *rays, ui
         if (!ctx || !gs || (count && (!rays || !hits))) fail(LR_INVALID, "a ray query needs rays and room for hits");
         if (count == 0) return;
         LR_CUDA(cudaSetDevice(ctx->device));
-        if (count <= kPadMost / 48 && pad_holds(ctx, count * 48)) {
+        if (count <= kPadMost / 48) {
+            std::lock_guard<std::recursive_mutex> turn(ctx->staging);
+            pad_hold(ctx, count * 48);
             char *d_hits = ctx->pad + count * 32;
             std::memcpy(ctx->pad_host, rays, count * 32);
             staged(ctx, [&] {

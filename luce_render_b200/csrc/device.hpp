@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 
 #include "common.hpp"
@@ -71,8 +72,9 @@ struct lr_context {
     unsigned long long *counts = nullptr;
     // Where small host-side queries stage their rays and results: device memory and page-locked
     // host memory of `pad_bytes` each (lr::kPadMost at most), made by the first such query, grown
-    // by a larger one, freed with the context; `words` holds the status words read back. Every
-    // query has waited for its work when it returns, and one thread drives a context.
+    // by a larger one, freed with the context; `words` holds the status words read back. A
+    // query holds `staging` until its results are out, so threads that share a context take turns.
+    std::recursive_mutex staging;
     char *pad = nullptr, *pad_host = nullptr;
     size_t pad_bytes = 0;
     int *words = nullptr;

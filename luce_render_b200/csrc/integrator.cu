@@ -1788,8 +1788,8 @@ bool wave_advance(WaveHost *h) {
 // all) and returns their paths a millisecond.
 double time_dry(WaveHost *h, int only, cudaEvent_t a, cudaEvent_t b) {
     // Warm: builds the variant's graph on every lane. (With one lane warmed, the other's capture
-    // fell between the events: rates of one variant a third of its neighbours', and a served
-    // stream tuned by them at 4.7 G pixel-samples/s instead of 6.3.)
+    // fell between the events, and some variants' rates came out a third of their neighbours';
+    // now they repeat within 2 %.)
     for (int i = 0; i < h->lane_count; i++) launch_pass(h, true, only);
     settle(h);
     uint64_t paths = 0;
