@@ -130,6 +130,9 @@ __device__ __forceinline__ bool watertight(const Shear &s, float tmin, float tma
     return true;
 }
 
+// An exit distance, or a hit's, as box entries are held against it: 1 + 2*gamma(3) times it.
+__device__ __forceinline__ float exit_slack(float t) { return t * 1.0000003576f; }
+
 // The slab test of the watertight path, one fused multiply-add per plane:
 // t = lo * inv + (-o * inv). The boxes are widened at upload by 2^-16 of the scene's
 // coordinate scale, which covers the rounding of this form (it moves a plane by at most
@@ -140,12 +143,11 @@ __device__ __forceinline__ bool watertight(const Shear &s, float tmin, float tma
 __device__ __forceinline__ bool box_exact(float lox, float hix, float loy, float hiy, float loz, float hiz,
                                           const float3 &inv, const float3 &oinv, float tmin, float tmax,
                                           float &enter) {
-    const float kScale = 1.0000003576f;
     const float x0 = fmaf(lox, inv.x, oinv.x), x1 = fmaf(hix, inv.x, oinv.x);
     const float y0 = fmaf(loy, inv.y, oinv.y), y1 = fmaf(hiy, inv.y, oinv.y);
     const float z0 = fmaf(loz, inv.z, oinv.z), z1 = fmaf(hiz, inv.z, oinv.z);
     const float e = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-    const float l = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax)) * kScale;
+    const float l = exit_slack(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), tmax)));
     enter = e;
     return e <= l;
 }
@@ -436,8 +438,8 @@ struct WideTracer {
                     for (int c = 0; c < 4; c++) {
                         const float e = fmax3(fmaf(nxs[c], inv.x, oinv.x), fmaf(nys[c], inv.y, oinv.y),
                                               fmaxf(fmaf(nzs[c], inv.z, oinv.z), r.tmin));
-                        const float l = fmin3(fmaf(fxs[c], inv.x, oinv.x), fmaf(fys[c], inv.y, oinv.y),
-                                              fminf(fmaf(fzs[c], inv.z, oinv.z), h.t)) * 1.0000003576f;
+                        const float l = exit_slack(fmin3(fmaf(fxs[c], inv.x, oinv.x), fmaf(fys[c], inv.y, oinv.y),
+                                                         fminf(fmaf(fzs[c], inv.z, oinv.z), h.t)));
                         key[p * 4 + c] = e <= l ? e : kMiss;
                         link[p * 4 + c] = ls[c];
                     }
@@ -490,7 +492,7 @@ struct WideTracer {
                 if (st.empty()) return true;
                 float t;
                 st.pop(node, t);
-                if (!(t > h.t)) break;
+                if (!(t > exit_slack(h.t))) break;
             }
         }
     }
@@ -568,8 +570,8 @@ struct CompressedTracer {
             const uint32_t nz = c < 4 ? nz0 : nz1, fz = c < 4 ? fz0 : fz1;
             const float e = fmax3(fmaf(byte_at(nx, k), ax, bx), fmaf(byte_at(ny, k), ay, by),
                                   fmaxf(fmaf(byte_at(nz, k), az, bz), r.tmin));
-            const float l = fmin3(fmaf(byte_at(fx, k), ax, bx), fmaf(byte_at(fy, k), ay, by),
-                                  fminf(fmaf(byte_at(fz, k), az, bz), h.t)) * 1.0000003576f;
+            const float l = exit_slack(fmin3(fmaf(byte_at(fx, k), ax, bx), fmaf(byte_at(fy, k), ay, by),
+                                             fminf(fmaf(byte_at(fz, k), az, bz), h.t)));
             mask |= e <= l ? 1u << c : 0u;
         }
         mask &= meta >> 24;  // occupied slots only

@@ -108,8 +108,9 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
                 bound = t;
             }
         }
-        // The children that are hit, the first group's nearest on top.
-        in = in && entry <= bound;
+        // The children that are hit, the first group's nearest on top. The same slack as the box
+        // test's: far from the scene an entry's rounding exceeds the boxes' widening.
+        in = in && entry <= exit_slack(bound);
         const uint32_t mask = __ballot_sync(kAll, in);
         const uint32_t ranks = octant_ranks((mask >> (8u * group)) & 0xffu, oct);
         const uint32_t above = (group == 3u ? 0u : (uint32_t)__popc(mask >> (8u * group + 8u))) +
