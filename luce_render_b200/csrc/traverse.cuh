@@ -62,6 +62,12 @@ __device__ __forceinline__ float3 safe_inverse(float3 d) {
     return make_float3(one(d.x), one(d.y), one(d.z));
 }
 
+// The next float above t, of either sign (above either zero: the smallest denormal).
+__device__ __forceinline__ float next_above(float t) {
+    const int bits = __float_as_int(fadd_(t, 0.0f));
+    return __int_as_float(bits + ((bits >> 31) | 1));
+}
+
 // The ray's shear for the watertight test: kz the largest |d| component (the first on
 // ties), kx and ky the next two (swapped when d[kz] < 0).
 struct Shear {
@@ -246,6 +252,7 @@ struct ExactTracer {
     float3 inv, oinv;
     Shear sh;
     Hit h;
+    float limit;  // triangles hit before it: r.tmax, then just past h.t (equal t may win on a smaller id)
     int node;
     SharedStack<kStack> st;
 
@@ -256,6 +263,7 @@ struct ExactTracer {
         const DeviceBvh &b = s.bvh;
         r = ray;
         h = Hit{r.tmax, -1, -1, 0.0f, 0.0f};
+        limit = r.tmax;
         st.sp = 0;
         if (b.empty) return false;
         inv = safe_inverse(r.d);
@@ -303,13 +311,12 @@ struct ExactTracer {
         for (uint32_t i = 0; i < count; i++) {
             const float4 *tri = s.tris + (size_t)(first + i) * 3;
             const float4 a = __ldg(tri), bb = __ldg(tri + 1), c = __ldg(tri + 2);
-            // Equal t may still win on a smaller id: test up to the next float above h.t.
-            const float limit = h.id >= 0 ? __int_as_float(__float_as_int(h.t) + 1) : r.tmax;
             float t, u, v;
             if (!watertight(sh, r.tmin, limit, a, bb, c, t, u, v)) continue;
             const int id = __float_as_int(a.w);
             if (h.id >= 0 && t == h.t && id > h.id) continue;
             h.t = t;
+            limit = next_above(t);
             h.id = id;
             h.slot = (int)(first + i);
             h.u = u;
@@ -376,6 +383,7 @@ struct WideTracer {
     float3 inv, oinv;
     Shear sh;
     Hit h;
+    float limit;  // as ExactTracer's
     int node;
     PairStack<kStack> st;
 
@@ -384,6 +392,7 @@ struct WideTracer {
     __device__ __forceinline__ bool start(const DeviceScene &s, const Ray &ray) {
         r = ray;
         h = Hit{r.tmax, -1, -1, 0.0f, 0.0f};
+        limit = r.tmax;
         st.sp = 0;
         const DeviceBvh &b = s.bvh;
         if (b.empty) return false;
@@ -474,12 +483,12 @@ struct WideTracer {
                 for (uint32_t i = 0; i < count; i++) {
                     const float4 *tri = s.tris + (size_t)(first + i) * 3;
                     const float4 a = __ldg(tri), bb = __ldg(tri + 1), c = __ldg(tri + 2);
-                    const float limit = h.id >= 0 ? __int_as_float(__float_as_int(h.t) + 1) : r.tmax;
                     float t, u, v;
                     if (!watertight(sh, r.tmin, limit, a, bb, c, t, u, v)) continue;
                     const int id = __float_as_int(a.w);
                     if (h.id >= 0 && t == h.t && id > h.id) continue;
                     h.t = t;
+                    limit = next_above(t);
                     h.id = id;
                     h.slot = (int)(first + i);
                     h.u = u;
@@ -513,6 +522,7 @@ struct CompressedTracer {
     float3 inv, oinv;
     Shear sh;
     Hit h;
+    float limit;   // as ExactTracer's
     uint32_t oct;  // bit k: the direction's component k is negative (its inverse, here)
     int *base;
     int stride;
@@ -523,6 +533,7 @@ struct CompressedTracer {
     __device__ __forceinline__ bool start(const DeviceScene &s, const Ray &ray) {
         r = ray;
         h = Hit{r.tmax, -1, -1, 0.0f, 0.0f};
+        limit = r.tmax;
         sp = 0;
         const DeviceBvh &b = s.bvh;
         if (b.empty) return false;
@@ -627,12 +638,12 @@ struct CompressedTracer {
                 for (uint32_t i = 0; i < count; i++) {
                     const float4 *tri = s.tris + (size_t)(first + i) * 3;
                     const float4 a = __ldg(tri), bb = __ldg(tri + 1), c = __ldg(tri + 2);
-                    const float limit = h.id >= 0 ? __int_as_float(__float_as_int(h.t) + 1) : r.tmax;
                     float t, u, v;
                     if (!watertight(sh, r.tmin, limit, a, bb, c, t, u, v)) continue;
                     const int id = __float_as_int(a.w);
                     if (h.id >= 0 && t == h.t && id > h.id) continue;
                     h.t = t;
+                    limit = next_above(t);
                     h.id = id;
                     h.slot = (int)(first + i);
                     h.u = u;

@@ -83,7 +83,7 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
         bool in = node && box_exact(p.x, q.x, p.y, q.y, p.z, q.z, inv, oinv, r.tmin, bound, entry) && q.w != 0.0f;
         if (__any_sync(kAll, leaf)) {
             bool better = false;
-            const float limit = found ? __int_as_float(__float_as_int(bound) + 1) : r.tmax;
+            const float limit = found ? next_above(bound) : r.tmax;
             for (uint32_t i = c; i < n; i += 8u) {
                 float4 a = p, b = q, d = v2;
                 if (i >= 8u) {
@@ -106,11 +106,12 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
 #pragma unroll
                 for (int step = 16; step > 0; step >>= 1) t = fminf(t, __shfl_xor_sync(kAll, t, step));
                 bound = t;
+                // Against this step's hits too, with the box test's slack: far from the scene an
+                // entry's rounding exceeds the boxes' widening.
+                in = in && entry <= exit_slack(bound);
             }
         }
-        // The children that are hit, the first group's nearest on top. The same slack as the box
-        // test's: far from the scene an entry's rounding exceeds the boxes' widening.
-        in = in && entry <= exit_slack(bound);
+        // The children that are hit, the first group's nearest on top.
         const uint32_t mask = __ballot_sync(kAll, in);
         const uint32_t ranks = octant_ranks((mask >> (8u * group)) & 0xffu, oct);
         const uint32_t above = (group == 3u ? 0u : (uint32_t)__popc(mask >> (8u * group + 8u))) +
