@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kBlock) trace_resident_kernel(DeviceScene s, c
     bool overflow = false;
     Visits visits;
     auto load = [&](uint32_t i) {
-        const float4 a = __ldg(&rays[2 * i]), b = __ldg(&rays[2 * i + 1]);
+        const float4 a = __ldg(&rays[2 * (size_t)i]), b = __ldg(&rays[2 * (size_t)i + 1]);
         return Ray{make_float3(a.x, a.y, a.z), a.w, make_float3(b.x, b.y, b.z), b.w};
     };
     auto store = [&](uint32_t i, const Hit &h, const Ray &) {
