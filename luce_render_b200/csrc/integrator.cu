@@ -980,9 +980,14 @@ Graph &finish_graph(WaveHost *h, Lane &lane, int stage) {
     return lane.finish.emplace(stage, g).first->second;
 }
 
-// Each lane's plain film stage as a graph.
-void lanes_capture(WaveHost *h) {
-    for (int li = 0; li < h->lane_count; li++) finish_graph(h, h->lanes[li], 0);
+// Makes every lane's graphs of the film stages a pass can reach (`folds`, `adapts`: whether some
+// pass may fold splats or check convergence), so that no pass has to: one takes 90 us.
+void prepare_film(WaveHost *h, bool folds, bool adapts) {
+    if (h->profile) return;  // launched by kernel
+    const int most = (folds ? kFilmFolds : 0) | (adapts ? kFilmAdapts : 0);
+    for (int stage = 0; stage <= most; stage++)
+        if ((stage & most) == stage)
+            for (int li = 0; li < h->lane_count; li++) finish_graph(h, h->lanes[li], stage);
 }
 
 void wave_create(WaveHost *h, lr_context *ctx, uint64_t pool, uint32_t rounds, uint32_t capacity, int profile) {
@@ -1039,8 +1044,6 @@ void wave_create(WaveHost *h, lr_context *ctx, uint64_t pool, uint32_t rounds, u
     h->grid_shade_glossy = grid_of(shade_kernel<false, true, false>, kShadeBlock, ctx->sm_count);
     if (profile)
         for (auto &e : h->mark_start) LR_CUDA(cudaEventCreate(&e));
-    else
-        lanes_capture(h);
     h->members.resize(capacity);
 }
 
@@ -1992,7 +1995,6 @@ void wave_resize(WaveHost *h, uint64_t pool, uint32_t rounds) {
     h->rounds = rounds;
     lanes_create(h);
     LR_CUDA(cudaStreamSynchronize(h->ctx->stream));
-    if (!h->profile) lanes_capture(h);
 }
 
 void wave_destroy(WaveHost *h) {
@@ -2240,6 +2242,7 @@ void renderer_renew(lr_renderer *r, const lr_frame &frame, const lr_scene *scene
     if (band + most_lights > h->pool || rounds > h->rounds)
         wave_resize(h, std::max<uint64_t>(band + most_lights, h->pool), std::max(rounds, h->rounds));
     member_renew(h, 0, frame, scene, settings, gs, gs);
+    prepare_film(h, h->members[0].dev.light_paths != 0u, h->members[0].dev.half != nullptr);
     r->bands = (uint32_t)((pixels + band - 1) / band);
     h->fill = (uint32_t)std::min<uint64_t>(band + h->members[0].dev.light_paths, h->pool);
     h->camera_cap = (uint32_t)band;
@@ -2263,6 +2266,7 @@ void create(lr_context *ctx, const lr_scene *scene, const lr_settings &settings,
         const uint32_t rounds = settings.max_bounces + 1 + (has_cutouts(*scene, settings) ? kCutoutRounds : 0);
         wave_create(&r->wave, ctx, band + most_lights, rounds, 1, settings.profile);
         member_add(&r->wave, gs, gs, scene, settings, frame);
+        prepare_film(&r->wave, r->wave.members[0].dev.light_paths != 0u, r->wave.members[0].dev.half != nullptr);
         r->wave.fill = (uint32_t)std::min<uint64_t>(band + r->wave.members[0].dev.light_paths, r->wave.pool);
         r->wave.camera_cap = (uint32_t)band;
         display_images(&r->wave, pixels);
@@ -2634,6 +2638,7 @@ int lr_batch_create(lr_context *ctx, const lr_batch_settings *settings, lr_batch
         auto b = std::make_unique<lr_batch>();
         try {
             wave_create(&b->wave, ctx, settings->pool, settings->max_bounces + 1, settings->capacity, settings->profile);
+            prepare_film(&b->wave, true, true);  // whatever its members will ask for
         } catch (...) {
             wave_destroy(&b->wave);
             throw;
