@@ -670,7 +670,6 @@ int lr_gpu_scene_upload(lr_context *ctx, const lr_scene *scene, lr_gpu_scene **o
         for (auto &p : parts)
             if (p.bytes && p.src)
                 LR_CUDA(cudaMemcpyAsync(base + p.offset, p.src, p.bytes, cudaMemcpyHostToDevice, ctx->stream));
-        LR_CUDA(cudaStreamSynchronize(ctx->stream));
         DeviceScene &s = gs->scene;
         s.bvh.entries = (const float4 *)(base + parts[0].offset);
         s.ref_bvh.entries = (const float4 *)(base + parts[1].offset);

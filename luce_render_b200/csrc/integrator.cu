@@ -633,8 +633,45 @@ struct Lane {
     uint64_t reads_seen = 0;         // the image reads its film stage has waited for
 };
 
+// The streams that a wave's graphs are captured on, a pass's work and what it forks beside it,
+// and the events of the forks and joins: made by the first capture and kept for the next, as a
+// stream made and destroyed takes 110 us, as long as a graph's capture and instantiation.
+struct Fork {
+    cudaStream_t main = nullptr, side = nullptr;
+    std::vector<cudaEvent_t> events;
+    size_t used = 0;  // of the events, in the capture under way
+    Fork() = default;
+    Fork(const Fork &) = delete;
+    Fork &operator=(const Fork &) = delete;
+    ~Fork() { release(); }
+    void release() {
+        for (cudaEvent_t e : events) cudaEventDestroy(e);
+        events.clear();
+        if (side) cudaStreamDestroy(side);
+        if (main) cudaStreamDestroy(main);
+        main = side = nullptr;
+    }
+    void begin() {
+        for (cudaStream_t *s : {&main, &side})
+            if (!*s) LR_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+        used = 0;
+    }
+    // Work queued on `to` from here on follows what is queued on `from` so far.
+    void order(cudaStream_t from, cudaStream_t to) {
+        if (used == events.size()) {
+            cudaEvent_t e;
+            LR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            events.push_back(e);
+        }
+        LR_CUDA(cudaEventRecord(events[used], from));
+        LR_CUDA(cudaStreamWaitEvent(to, events[used], 0));
+        used++;
+    }
+};
+
 struct WaveHost {
     lr_context *ctx = nullptr;
+    Fork fork;  // what its graphs are captured with
     uint32_t pool = 0, rounds = 0, capacity = 0;
     int profile = 0;
     void *block = nullptr;  // the member table and stats, shared by the lanes
@@ -719,28 +756,6 @@ void mark(cudaStream_t stream, Marks *marks, int kind) {
     marks->push_back({e, kind});
 }
 
-// A side stream that a captured pass forks part of its work onto, and the events of the
-// forks and joins; they live until the capture ends.
-struct Fork {
-    cudaStream_t side = nullptr;
-    std::vector<cudaEvent_t> events;
-    Fork() { LR_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking)); }
-    Fork(const Fork &) = delete;
-    Fork &operator=(const Fork &) = delete;
-    ~Fork() {
-        for (cudaEvent_t e : events) cudaEventDestroy(e);
-        cudaStreamDestroy(side);
-    }
-    // Work queued on `to` from here on follows what is queued on `from` so far.
-    void order(cudaStream_t from, cudaStream_t to) {
-        cudaEvent_t e;
-        LR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        events.push_back(e);
-        LR_CUDA(cudaEventRecord(e, from));
-        LR_CUDA(cudaStreamWaitEvent(to, e, 0));
-    }
-};
-
 // Records a pass's tracing on `stream` with traversal (width, stack entries) in blocks of
 // `block` threads: camera, then (closest, shade, shadow) for every round. With `marks`,
 // an event follows each kernel (profiling); `count` takes the counting traversals.
@@ -757,17 +772,22 @@ struct Fork {
 // triangles 1,713 -> 1,370 us, glossy box with light tracing 512x500 x 2 3,775 -> 3,234 us,
 // 1080p of 1M triangles x 4 13.85 -> 13.09 ms (thick rounds fill the machine either way; what
 // is left to gain there is the tails).
+//
+// Without light paths it is the closest hits that go to the side stream and the shadow rays that
+// stay: the same graph, but instantiating it takes 150 us where the other way round takes 440 (22
+// nodes; why is the driver's). With light paths the side holds their shading and the shadow rays.
 void record_trace(const WaveHost *h, const Wave &w, int width, int stack, int block, bool count, bool refill,
                   int grid_trace, bool tracing, bool glossy, bool cutouts, cudaStream_t stream, Marks *marks,
                   int thin_stack, int thin_grid, Fork *fork) {
     cudaStream_t side = fork ? fork->side : stream;
+    cudaStream_t shadows = tracing ? side : stream;
     camera_kernel<<<h->grid_shade, kShadeBlock, 0, stream>>>(w);
     mark(stream, marks, kCamera);
     for (uint32_t round = 0; round < w.rounds; round++) {
         // From round thin_from on (thin queues, latency-bound) the compressed 8-wide tree.
         const bool thin = thin_stack && (int)round >= h->thin_from;
         const int rw = thin ? 8 : width, rs = thin ? thin_stack : stack, rg = thin ? thin_grid : grid_trace;
-        launch_closest(rw, rs, block, count, refill, rg, stream, w, round);
+        launch_closest(rw, rs, block, count, refill, rg, round > 0 && !tracing ? side : stream, w, round);
         mark(stream, marks, kClosest);
         if (fork && round > 0) fork->order(side, stream);
         if (fork && tracing) fork->order(stream, side);
@@ -787,7 +807,7 @@ void record_trace(const WaveHost *h, const Wave &w, int width, int stack, int bl
         mark(stream, marks, kSurface);
         if (fork && tracing) fork->order(side, stream);
         if (fork) fork->order(stream, side);
-        launch_shadow(rw, rs, block, count, cutouts, refill, rg, side, w, round);
+        launch_shadow(rw, rs, block, count, cutouts, refill, rg, shadows, w, round);
         mark(stream, marks, kShadow);
     }
     if (fork) fork->order(side, stream);
@@ -863,16 +883,22 @@ void record_trace_any(WaveHost *h, const Wave &w, int variant, cudaStream_t stre
                  thin_stack, thin_grid, fork);
 }
 
-// Captures whatever `body` queues on a private stream as a graph.
+// Captures whatever `body` queues on the fork's streams as a graph.
 template <class Body>
-Graph capture(Body body) {
+Graph capture(Fork &fork, Body body) {
     Graph g;
-    cudaStream_t stream;
-    LR_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    LR_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    body(stream);
-    LR_CUDA(cudaStreamEndCapture(stream, &g.graph));
-    LR_CUDA(cudaStreamDestroy(stream));
+    fork.begin();
+    LR_CUDA(cudaStreamBeginCapture(fork.main, cudaStreamCaptureModeThreadLocal));
+    try {
+        body(fork.main);
+    } catch (...) {
+        cudaGraph_t part = nullptr;
+        if (cudaStreamEndCapture(fork.main, &part) == cudaSuccess && part) cudaGraphDestroy(part);
+        cudaGetLastError();
+        fork.release();
+        throw;
+    }
+    LR_CUDA(cudaStreamEndCapture(fork.main, &g.graph));
     LR_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
     return g;
 }
@@ -881,8 +907,7 @@ Graph capture(Body body) {
 Graph &trace_graph(WaveHost *h, Lane &lane, int variant) {
     auto it = lane.trace.find(variant);
     if (it != lane.trace.end()) return it->second;
-    Fork fork;
-    Graph g = capture([&](cudaStream_t s) { record_trace_any(h, lane.w, variant, s, nullptr, &fork); });
+    Graph g = capture(h->fork, [&](cudaStream_t s) { record_trace_any(h, lane.w, variant, s, nullptr, &h->fork); });
     return lane.trace.emplace(variant, g).first->second;
 }
 
@@ -976,7 +1001,7 @@ void lanes_create(WaveHost *h) {
 Graph &finish_graph(WaveHost *h, Lane &lane, int stage) {
     auto it = lane.finish.find(stage);
     if (it != lane.finish.end()) return it->second;
-    Graph g = capture([&](cudaStream_t s) { record_finish(h, lane.w, stage, s, nullptr); });
+    Graph g = capture(h->fork, [&](cudaStream_t s) { record_finish(h, lane.w, stage, s, nullptr); });
     return lane.finish.emplace(stage, g).first->second;
 }
 
@@ -2023,6 +2048,7 @@ void wave_destroy(WaveHost *h) {
     if (h->display_block) cudaFree(h->display_block);
     h->display_block = nullptr;
     lanes_destroy(h);
+    h->fork.release();
     if (h->block) cudaFree(h->block);
 }
 
