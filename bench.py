@@ -51,7 +51,7 @@ def parse():
                    help="only the headline renderer's passes (--warmup, then --steps), for profiling; one JSON line")
     p.add_argument("--width", type=int, default=0, help="with --trace-only: the BVH width (2, 4, 8; 0 the default)")
     p.add_argument("--refill", type=int, default=-1,
-                   help="with --trace-only: idle lanes at which traversal warps refill (1-32; 0 grid-stride)")
+                   help="with --trace-only: idle lanes at which warps on wide trees refill (1-32; 0 warp batches)")
     p.add_argument("--cornell-only", action="store_true",
                    help="only the glossy Cornell benchmark lines (--steps samples each), one JSON line")
     p.add_argument("--served-seconds", type=float, default=60.0,

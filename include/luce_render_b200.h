@@ -555,7 +555,8 @@ typedef struct {
     uint32_t class_stack[3];   /* traversal stack entries chosen per size class */
     uint32_t class_block[3];   /* traversal kernels' threads a block chosen per size class */
     uint32_t bin_interval;     /* rounds between sorts of outgoing rays by octant (0: none) */
-    uint32_t refill_at;        /* idle lanes at which traversal warps refill (0: warp batches) */
+    uint32_t refill_at;        /* idle lanes at which warps on wide trees refill (0: warp batches, or no
+                                * wide tree is walked: the BVH2's warps refill by a rule of their own) */
     int32_t thin_from;         /* first round of a BVH2 pass on the compressed 8-wide tree (-1: none) */
 } lr_batch_tuning;
 int lr_batch_tune(lr_batch *batch, lr_batch_tuning *out);

@@ -1081,9 +1081,9 @@ class Batch:
 
     def tune(self) -> dict:
         """Autotune, per scene-size class, BVH width, traversal stack depth and threads a
-        block, then paths a pass, the interval of octant sorts of outgoing rays and the
-        traversal warps' refill point, on the members as they stand (images do not
-        change)."""
+        block, then paths a pass, the interval of octant sorts of outgoing rays and, where
+        a wide tree is walked, its warps' refill point, on the members as they stand
+        (images do not change)."""
         t = BatchTuning()
         _check(lib.lr_batch_tune(self.handle, C.byref(t)))
         return {"width": int(t.width), "fill": int(t.fill), "paths_per_ms": float(t.paths_per_ms),

@@ -710,8 +710,10 @@ struct WaveHost {
     // this (0: none). The wavefront compacts every round (warp- or block-aggregated
     // pushes); this is how often it also sorts.
     uint32_t bin_interval = 0;
-    // Idle lanes at which a traversal warp takes new queue entries (0: grid-stride walks).
+    // Idle lanes at which a warp that walks a wide tree takes new queue entries (0: warp
+    // batches). The BVH2's warps refill by their own rule (trace_bvh2).
     uint32_t refill_at = 0;
+    bool walks_wide = false;  // whether the pass planned last walks a wide tree in some round
     uint32_t fill = 0;
     // The most camera paths a pass takes (0: as many as fit): a renderer's band, so that
     // its passes are the reference's bands, light paths riding along in a sample's first.
@@ -1024,7 +1026,7 @@ void wave_create(WaveHost *h, lr_context *ctx, uint64_t pool, uint32_t rounds, u
     h->profile = profile;
     h->lane_count = profile ? 1 : 2;
     // The environment variable LUCE_RENDER_B200_REFILL (1 to 32) sets the idle lanes at
-    // which traversal warps refill until a tuner chooses, for measurement.
+    // which warps on wide trees refill until a tuner chooses, for measurement.
     if (const char *env = std::getenv("LUCE_RENDER_B200_REFILL")) {
         const int v = std::atoi(env);
         if (v >= 1 && v <= 32) h->refill_at = (uint32_t)v;
@@ -1700,11 +1702,13 @@ bool launch_pass(WaveHost *h, bool dry = false, int only = -1) {
     const bool walkable = std::all_of(rec.members.begin(), rec.members.end(), [&](const std::pair<uint32_t, bool> &e) {
         return warp_walkable(h->members[e.first].dev.scene, ints);
     });
+    h->walks_wide = width != 2 || thin != 0;
+    const uint32_t refill_at = h->walks_wide ? h->refill_at : 0u;
     const int variant = width * 1000 + stack + (tracing ? kTracingVariant : 0) + (glossy ? kGlossyVariant : 0) +
                         (cutouts ? kCutoutVariant : 0) + block_index * kBlockVariant +
-                        (h->refill_at ? kRefillVariant : 0) + thin * kThinVariant;
+                        (refill_at ? kRefillVariant : 0) + thin * kThinVariant;
     staging->head = PlanHeader{n, used, converts, dry ? 1u : 0u, camera_paths, folds, adapts, h->bin_interval,
-                               h->refill_at, walkable ? warp_rays_for(most_triangles) : 0u, vote_quarters(most_triangles), 0u};
+                               refill_at, walkable ? warp_rays_for(most_triangles) : 0u, vote_quarters(most_triangles), 0u};
     staging->display = PlanDisplay{0ull, h->display_scale, h->display_view, 0u, 0u};
     if (h->display_block && converts > 0) {
         rec.display_slot = free_display_slot(h);
@@ -1937,11 +1941,12 @@ void wave_tune(WaveHost *h, lr_batch_tuning *out) {
         }
     }
     h->bin_interval = best_interval;
-    // Persistent warps that refill their idle lanes from the queue, at 32 (a whole warp at
-    // a time), 16 or 8 idle lanes, against the grid-stride walks.
-    uint32_t best_refill = h->refill_at;
+    // On wide trees, persistent warps that refill their idle lanes from the queue, at 32 (a
+    // whole warp at a time), 16 or 8 idle lanes, against warp batches. Passes on the BVH2 alone
+    // have nothing to choose: every candidate would launch the same kernels.
+    uint32_t best_refill = h->walks_wide ? h->refill_at : 0u;
     for (uint32_t refill : {0u, 32u, 16u, 8u}) {
-        if (refill == h->refill_at) continue;
+        if (!h->walks_wide || refill == h->refill_at) continue;
         const uint32_t kept = h->refill_at;
         h->refill_at = refill;
         const double rate = time_dry(h, -1, a, b);
@@ -1959,6 +1964,7 @@ void wave_tune(WaveHost *h, lr_batch_tuning *out) {
     h->thin_any = true;
     int best_thin = -1;
     double best_thin_rate = -1.0;
+    bool best_wide = false;
     for (int from : {-1, 2, 3, 4}) {
         h->thin_from = from;
         const double rate = time_dry(h, -1, a, b);
@@ -1966,9 +1972,11 @@ void wave_tune(WaveHost *h, lr_batch_tuning *out) {
         if (rate > best_thin_rate) {
             best_thin_rate = rate;
             best_thin = from;
+            best_wide = h->walks_wide;
         }
     }
     h->thin_from = best_thin;
+    if (!best_wide) h->refill_at = best_refill = 0;  // its wide rounds went with the choice
     best = std::max(best, best_thin_rate);
     cudaEventDestroy(a);
     cudaEventDestroy(b);
@@ -2301,17 +2309,16 @@ void create(lr_context *ctx, const lr_scene *scene, const lr_settings &settings,
         r->shading = scene->shading;
         // The graphs for the scene's traversal variant, made now rather than at the first pass.
         const TraversalChoice c = choose_traversal(gs->scene, 0);
+        const bool thins = r->wave.thin_from >= 0 && c.width == 2 &&
+                           (r->wave.thin_any || size_class(gs->scene.triangle_count) == kSizeClasses - 1);
+        const int thin = thins ? thin_code(gs->scene) : 0;
         if (!settings.profile)
             for (int li = 0; li < r->wave.lane_count; li++)
                 trace_graph(&r->wave, r->wave.lanes[li],
                             c.width * 1000 + c.stack + (r->wave.members[0].dev.light_paths ? kTracingVariant : 0) +
                                 (r->wave.members[0].dev.glossy ? kGlossyVariant : 0) +
                                 (r->wave.members[0].dev.cutouts ? kCutoutVariant : 0) +
-                                (r->wave.refill_at ? kRefillVariant : 0) +
-                                (r->wave.thin_from >= 0 && c.width == 2 && r->wave.profile < 2 &&
-                                         size_class(gs->scene.triangle_count) == kSizeClasses - 1
-                                     ? thin_code(gs->scene) * kThinVariant
-                                     : 0));
+                                (r->wave.refill_at && (c.width != 2 || thin) ? kRefillVariant : 0) + thin * kThinVariant);
     } catch (...) {
         const bool owned = !r->wave.members.empty() && r->wave.members[0].used;
         wave_destroy(&r->wave);

@@ -384,7 +384,7 @@ void render_loop(lr_server *s) {
         if (retune) {
             // Dry passes on the live sessions (films untouched): the BVH width, stack and
             // block size per scene-size class, the pass fill, the ray sort interval and
-            // the traversal warps' refill.
+            // the wide trees' refill.
             t = Clock::now();
             const bool tuned = lr_batch_tune(s->batch, nullptr) == LR_OK;
             std::lock_guard<std::mutex> note(s->mu);

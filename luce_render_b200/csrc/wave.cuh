@@ -94,8 +94,8 @@ struct PlanHeader {
     // bin_interval: the shade kernels group outgoing rays by direction octant in rounds
     // that are multiples of it (0: never; an autotuner choice).
     uint32_t camera_paths, folds, adapts, bin_interval;
-    // refill_at: the traversal kernels' persistent warps take new queue entries once this
-    // many of their lanes are idle (1 to 32; 0: grid-stride walks; an autotuner choice).
+    // refill_at: on a wide tree the traversal kernels' persistent warps take new queue entries
+    // once this many of their lanes are idle (1 to 32; 0: warp batches; an autotuner choice).
     // warp_rays: queues of at most this many rays a warp of the launch are walked a warp a
     // ray (warpwalk.cuh; 0: none, some member's tree cannot be).
     // vote_quarters: trace_bvh2's, for the member with most of the pass's paths.
