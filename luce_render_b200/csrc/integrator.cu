@@ -780,14 +780,14 @@ void mark(cudaStream_t stream, Marks *marks, int kind) {
 // nodes; why is the driver's). With light paths the side holds their shading and the shadow rays.
 void record_trace(const WaveHost *h, const Wave &w, int width, int stack, int block, bool count, bool refill,
                   int grid_trace, bool tracing, bool glossy, bool cutouts, cudaStream_t stream, Marks *marks,
-                  int thin_stack, int thin_grid, Fork *fork) {
+                  int thin_stack, int thin_grid, int thin_from, Fork *fork) {
     cudaStream_t side = fork ? fork->side : stream;
     cudaStream_t shadows = tracing ? side : stream;
     camera_kernel<<<h->grid_shade, kShadeBlock, 0, stream>>>(w);
     mark(stream, marks, kCamera);
     for (uint32_t round = 0; round < w.rounds; round++) {
         // From round thin_from on (thin queues, latency-bound) the compressed 8-wide tree.
-        const bool thin = thin_stack && (int)round >= h->thin_from;
+        const bool thin = thin_stack && (int)round >= thin_from;
         const int rw = thin ? 8 : width, rs = thin ? thin_stack : stack, rg = thin ? thin_grid : grid_trace;
         launch_closest(rw, rs, block, count, refill, rg, round > 0 && !tracing ? side : stream, w, round);
         mark(stream, marks, kClosest);
@@ -846,10 +846,26 @@ constexpr int kTraceBlocks[3] = {kTraceBlock, 64, 256};
 // when it holds light tracing, kGlossyVariant when it holds glossy materials,
 // kCutoutVariant when it holds cut-outs, kBlockVariant times the index of the traversal
 // kernels' block size in kTraceBlocks, kRefillVariant when its traversal warps refill
-// idle lanes from the queue, and kThinVariant times 1 or 2 when its later rounds walk the
-// compressed 8-wide tree with 16 or 32 group entries.
+// idle lanes from the queue, and thin_variant when its later rounds walk the compressed
+// 8-wide tree: with 16 or 32 group entries (thin code 1 or 2), from round `from` on.
 constexpr int kTracingVariant = 100000, kGlossyVariant = 200000, kCutoutVariant = 400000, kBlockVariant = 800000,
               kRefillVariant = 3 * kBlockVariant, kThinVariant = 2 * kRefillVariant;
+constexpr int kThinRounds = 16;  // the first thin round is one of these
+
+constexpr int thin_variant(int code, int from) { return code ? (2 * from + code) * kThinVariant : 0; }
+constexpr int thin_code_of(int variant) { return variant < kThinVariant ? 0 : 1 + (variant / kThinVariant - 1) % 2; }
+constexpr int thin_from_of(int variant) { return (variant / kThinVariant - 1) / 2; }
+static_assert((2 * kThinRounds + 1LL) * kThinVariant <= 0x7fffffffLL, "a variant is an int");
+// A graph is kept by its variant, and holds its first thin round.
+constexpr bool thin_variants_differ() {
+    for (int from = 0; from < kThinRounds; from++)
+        for (int code = 1; code <= 2; code++) {
+            const int v = thin_variant(code, from) + kThinVariant - 1;
+            if (thin_code_of(v) != code || thin_from_of(v) != from) return false;
+        }
+    return thin_code_of(kThinVariant - 1) == 0;
+}
+static_assert(thin_variants_differ(), "a variant tells its first thin round");
 
 int variant_block(int variant) { return kTraceBlocks[(variant / kBlockVariant) % 3]; }
 
@@ -878,11 +894,11 @@ void record_trace_any(WaveHost *h, const Wave &w, int variant, cudaStream_t stre
     const int width = traversal / 1000, stack = traversal % 1000, block = variant_block(variant);
     const bool count = h->profile >= 2, refill = ((variant / kRefillVariant) & 1) && !count;
     const int grid = grid_for(h, width, stack, block, refill);
-    const int thin = variant / kThinVariant;  // 0: none; 1, 2: the 8-wide tree with 16, 32 groups
+    const int thin = thin_code_of(variant);
     const int thin_stack = thin == 1 ? 16 : (thin == 2 ? 32 : 0);
     const int thin_grid = thin_stack ? grid_for(h, 8, thin_stack, block, refill) : 0;
     record_trace(h, w, width, stack, block, count, refill, grid, flags & 1, flags & 2, flags & 4, stream, marks,
-                 thin_stack, thin_grid, fork);
+                 thin_stack, thin_grid, thin_from_of(variant), fork);
 }
 
 // Captures whatever `body` queues on the fork's streams as a graph.
@@ -1035,7 +1051,7 @@ void wave_create(WaveHost *h, lr_context *ctx, uint64_t pool, uint32_t rounds, u
     // mix of members, for measurement.
     if (const char *env = std::getenv("LUCE_RENDER_B200_THIN")) {
         const int v = std::atoi(env);
-        if (v >= -1 && v <= 15) {
+        if (v >= -1 && v < kThinRounds) {
             h->thin_from = v;
             h->thin_any = true;
         }
@@ -1706,7 +1722,7 @@ bool launch_pass(WaveHost *h, bool dry = false, int only = -1) {
     const uint32_t refill_at = h->walks_wide ? h->refill_at : 0u;
     const int variant = width * 1000 + stack + (tracing ? kTracingVariant : 0) + (glossy ? kGlossyVariant : 0) +
                         (cutouts ? kCutoutVariant : 0) + block_index * kBlockVariant +
-                        (refill_at ? kRefillVariant : 0) + thin * kThinVariant;
+                        (refill_at ? kRefillVariant : 0) + thin_variant(thin, h->thin_from);
     staging->head = PlanHeader{n, used, converts, dry ? 1u : 0u, camera_paths, folds, adapts, h->bin_interval,
                                refill_at, walkable ? warp_rays_for(most_triangles) : 0u, vote_quarters(most_triangles), 0u};
     staging->display = PlanDisplay{0ull, h->display_scale, h->display_view, 0u, 0u};
@@ -2318,7 +2334,8 @@ void create(lr_context *ctx, const lr_scene *scene, const lr_settings &settings,
                             c.width * 1000 + c.stack + (r->wave.members[0].dev.light_paths ? kTracingVariant : 0) +
                                 (r->wave.members[0].dev.glossy ? kGlossyVariant : 0) +
                                 (r->wave.members[0].dev.cutouts ? kCutoutVariant : 0) +
-                                (r->wave.refill_at && (c.width != 2 || thin) ? kRefillVariant : 0) + thin * kThinVariant);
+                                (r->wave.refill_at && (c.width != 2 || thin) ? kRefillVariant : 0) +
+                                thin_variant(thin, r->wave.thin_from));
     } catch (...) {
         const bool owned = !r->wave.members.empty() && r->wave.members[0].used;
         wave_destroy(&r->wave);
