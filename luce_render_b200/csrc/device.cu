@@ -1,6 +1,7 @@
 // The context, the scene in HBM (GpuScene.upload, src/render/device.lucb:41-89), the
 // primary-ray probe (device.lucb:138-160, shaders/probe.comp) and ray-list queries.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -187,44 +188,41 @@ TraversalChoice choose_traversal(const DeviceScene &s, int requested) {
 
 namespace {
 
+// The blocks of a kernel that the current device holds at once, worked out on each device's first
+// launch of it (by any thread: they agree).
+template <auto kKernel>
+unsigned resident_blocks() {
+    static std::atomic<unsigned> known[64];
+    int device = 0;
+    LR_CUDA(cudaGetDevice(&device));
+    unsigned resident = device < 64 ? known[device].load(std::memory_order_relaxed) : 0u;
+    if (!resident) {
+        int per_sm = 0, sms = 0;
+        LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernel, kBlock, 0));
+        LR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        resident = (unsigned)(std::max(1, per_sm) * sms);
+        if (device < 64) known[device].store(resident, std::memory_order_relaxed);
+    }
+    return resident;
+}
+
 template <int W, bool kAny, int kStack, bool kCount>
 void launch_resident(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, float4 *hits, int *status,
                      unsigned long long *counts, cudaStream_t stream) {
-    static int resident = 0;
-    if (!resident) {
-        int per_sm = 0, device = 0, sms = 0;
-        LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_resident_kernel<W, kAny, kStack, kCount>,
-                                                              kBlock, 0));
-        LR_CUDA(cudaGetDevice(&device));
-        LR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        resident = std::max(1, per_sm) * sms;
-    }
+    const unsigned resident = resident_blocks<trace_resident_kernel<W, kAny, kStack, kCount>>();
     const uint64_t needed = (n + kBlock - 1) / kBlock;
-    const unsigned grid = (unsigned)std::min<uint64_t>(needed, (uint64_t)resident);
+    const unsigned grid = (unsigned)std::min<uint64_t>(needed, resident);
     uint32_t *next = (uint32_t *)(status + kBatchCursor);
     LR_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
     trace_resident_kernel<W, kAny, kStack, kCount><<<grid, kBlock, 0, stream>>>(gs->scene, rays, (uint32_t)n, hits,
                                                                                status, counts, next);
 }
 
-// The resident blocks of the warp-walk kernel on the current device.
-unsigned warps_resident() {
-    static int resident = 0;
-    if (!resident) {
-        int per_sm = 0, device = 0, sms = 0;
-        LR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_warps_kernel, kBlock, 0));
-        LR_CUDA(cudaGetDevice(&device));
-        LR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        resident = std::max(1, per_sm) * sms;
-    }
-    return (unsigned)resident;
-}
-
 // Short closest-hit queries of the default width a warp a ray: at most warp_rays_for rays a
 // resident warp, on a scene whose 8-wide tree fits the stack.
 bool launch_warps(const lr_gpu_scene *gs, const float4 *rays, uint64_t n, float4 *hits, int *status, cudaStream_t stream) {
     constexpr uint64_t kWarps = kBlock / 32;
-    const unsigned resident = warps_resident();
+    const unsigned resident = resident_blocks<trace_warps_kernel>();
     if (n > warp_rays_for(gs->scene.triangle_count) * kWarps * (uint64_t)resident || !warp_walkable(gs->scene, kWarpQueryInts)) return false;
     uint32_t *next = (uint32_t *)(status + kBatchCursor);
     LR_CUDA(cudaMemsetAsync(next, 0, sizeof(uint32_t), stream));
@@ -280,7 +278,7 @@ void dispatch_probe(const lr_gpu_scene *gs, const ProbeFrame &f, uint64_t count,
     // Up to two pixels a warp that fits the GPU: a camera's neighbouring rays keep a plain
     // warp's lanes in step, so the warp walk pays only while the frame cannot fill the GPU.
     constexpr uint64_t kWarps = kBlock / 32;
-    if (!kRef && count <= 2 * kWarps * warps_resident() && warp_walkable(gs->scene, kWarpQueryInts)) {
+    if (!kRef && count <= 2 * kWarps * resident_blocks<trace_warps_kernel>() && warp_walkable(gs->scene, kWarpQueryInts)) {
         probe_warps_kernel<<<(unsigned)((count + kWarps - 1) / kWarps), kBlock, 0, stream>>>(gs->scene, f, faces, ts, status);
         return;
     }
