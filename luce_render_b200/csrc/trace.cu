@@ -53,7 +53,7 @@ constexpr uint32_t kWarpInts = TracerOf<W, false, kStack, false>::kInts * 32u;
 // batch's rays decide (trace_bvh2). The shortest queues, on the BVH2 and the 8-wide tree, take
 // a warp a ray (walk_warp).
 template <int W, int kStack, bool kCount, bool kRefill>
-__device__ __forceinline__ void closest_body(const Wave &w, uint32_t round) {
+__global__ void __launch_bounds__(kTraceBlockMax, kTraceMinBlocks) closest_kernel(Wave w, uint32_t round) {
     extern __shared__ int stack[];  // kInts entries a thread, strided by the block's size
     const uint32_t q = round & 1u;
     const uint32_t cameras = w.counters[round], count = cameras + *light_counter(w, round);
@@ -127,11 +127,6 @@ __device__ __forceinline__ void closest_body(const Wave &w, uint32_t round) {
     }
     if (overflow) atomicAdd(&w.status[0], 1);
     if (kCount) add_visits(&w.stats[4], visits);
-}
-
-template <int W, int kStack, bool kCount, bool kRefill>
-__global__ void __launch_bounds__(kTraceBlockMax, kTraceMinBlocks) closest_kernel(Wave w, uint32_t round) {
-    closest_body<W, kStack, kCount, kRefill>(w, round);
 }
 
 // A shadow ray's hit id when its connection ended before the any-hit walk.
