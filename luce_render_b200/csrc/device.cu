@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kBlock) probe_kernel(DeviceScene s, ProbeFrame
 }
 
 // A warp a pixel, for small frames (warpwalk.cuh): their launch has a block for every four.
-__global__ void __launch_bounds__(kBlock) probe_warps_kernel(DeviceScene s, ProbeFrame f, uint32_t *faces, float *ts,
+__global__ void __launch_bounds__(kBlock, 7) probe_warps_kernel(DeviceScene s, ProbeFrame f, uint32_t *faces, float *ts,
                                                             int *status) {
     __shared__ int stack[kBlock / 32][kWarpQueryInts];
     const uint64_t pixel = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(kBlock) trace_resident_kernel(DeviceScene s, c
 }
 
 // Closest hits of a short ray list, a warp a ray (warpwalk.cuh). An any-hit query reports the
-// hit it finds first, which is the BVH2 walk's, and does not come here.
-__global__ void __launch_bounds__(kBlock) trace_warps_kernel(DeviceScene s, const float4 *__restrict__ rays, uint32_t n,
+// hit it finds first, which is the BVH2 walk's, and does not come here. Seven blocks an SM are the
+// 72 registers the walk needs; unbounded the compiler takes 64 and spills (1 % of a call).
+__global__ void __launch_bounds__(kBlock, 7) trace_warps_kernel(DeviceScene s, const float4 *__restrict__ rays, uint32_t n,
                                                             float4 *__restrict__ hits, int *status, uint32_t *next) {
     __shared__ int stack[kBlock / 32][kWarpQueryInts];
     bool overflow = false;

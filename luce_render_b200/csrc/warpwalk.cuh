@@ -63,6 +63,7 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
     const Shear sh = make_shear(r.o, r.d);
     const uint32_t oct = (inv.x < 0.0f ? 1u : 0u) | (inv.y < 0.0f ? 2u : 0u) | (inv.z < 0.0f ? 4u : 0u);
     float bound = r.tmax;  // the nearest hit so far
+    float limit = r.tmax;  // triangles hit before it, as ExactTracer's
     bool found = false;
     uint32_t sp = 0, taken = 1;
     int link = 0;  // this group's entry when group < taken: the root first
@@ -83,7 +84,6 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
         bool in = node && box_exact(p.x, q.x, p.y, q.y, p.z, q.z, inv, oinv, r.tmin, bound, entry) && q.w != 0.0f;
         if (__any_sync(kAll, leaf)) {
             bool better = false;
-            const float limit = found ? next_above(bound) : r.tmax;
             for (uint32_t i = c; i < n; i += 8u) {
                 float4 a = p, b = q, d = v2;
                 if (i >= 8u) {
@@ -106,6 +106,7 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
 #pragma unroll
                 for (int step = 16; step > 0; step >>= 1) t = fminf(t, __shfl_xor_sync(kAll, t, step));
                 bound = t;
+                limit = next_above(t);
                 // Against this step's hits too, with the box test's slack: far from the scene an
                 // entry's rounding exceeds the boxes' widening.
                 in = in && entry <= exit_slack(bound);
