@@ -807,11 +807,12 @@ def main():
     roofline = {
         "kernel": "closest_kernel (intersect closest)",
         # The scene (~100 MB) stays in the 126 MB L2: DRAM moves a few percent of the
-        # algorithmic bytes, and the kernel waits on L1/L2 latency with few lanes of a
-        # warp active (divergent incoherent traversal). Reported against HBM as the
-        # roofline asks; the bound the counters show is latency.
+        # algorithmic bytes and is used at 3.6 %, so a fraction of HBM says how fast the
+        # algorithm's bytes are served, not how busy HBM is. Reported against HBM as the
+        # roofline asks; the counters show L1's data pipe at 89 % of its wavefronts on long
+        # queues (a lane of a divergent load is one), dependent fetches on short ones.
         "bound": "hbm",
-        "bound_observed": "latency (L2-resident scene; divergent traversal; ncu summary in profiles/)",
+        "bound_observed": "L1 data pipe (long queues; L2-resident scene, HBM at 3.6 %; ncu summary in profiles/)",
         "achieved": achieved,
         "peak": hbm if hbm else 6650.0,
         "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if hbm else "fallback 6.65 TB/s",
@@ -912,8 +913,8 @@ def main():
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": "Mrays/s", "h2d_bytes_per_step": 0,
                     "d2h_bytes_per_step": WIDTH * HEIGHT * 16},
-            # a pass: camera; closest, shade and shadow each round; finish, fold, the two
-            # adaptive phases and convert (the launch list in profiles/ counts the same)
+            # a pass: camera; closest, shade and shadow each round; finish and convert (no
+            # splats to fold, no convergence to check; the launch list in profiles/ counts the same)
             "gpu_launches": K * (1 + 3 * (BOUNCES + 1) + 2),
             "clocks": clock_info,
             "light_traced": traced_info,

@@ -73,7 +73,9 @@ struct lr_context {
     // Where small host-side queries stage their rays and results: device memory and page-locked
     // host memory of `pad_bytes` each (lr::kPadMost at most), made by the first such query, grown
     // by a larger one, freed with the context; `words` holds the status words read back. A
-    // query holds `staging` until its results are out, so threads that share a context take turns.
+    // small query holds `staging` until its results are out, and check_status while it reads the
+    // words. That guards these buffers alone: a context is one thread's at a time (its larger
+    // and device-resident queries share a batch cursor and status words and take no lock).
     std::recursive_mutex staging;
     char *pad = nullptr, *pad_host = nullptr;
     size_t pad_bytes = 0;

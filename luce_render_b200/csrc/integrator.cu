@@ -681,12 +681,15 @@ struct WaveHost {
     // its members have one (-1: every round on the BVH2). The first rounds hold most of a
     // pass's rays and the BVH2 traces them fastest; later rounds hold few, and each is as
     // long as its slowest rays' chains of dependent node fetches, which the 8-wide tree
-    // shortens (measured: from round 3, 1,313 against 1,284-1,291 Mrays/s on the headline
-    // pass; from round 2 1,294, from round 4 1,298-1,303).
+    // shortens. Most such queues are walked a warp a ray on either tree (warpwalk.cuh); for the
+    // ones between, four samples from round 3 on, against every round on the BVH2, from
+    // round 2 and from round 4 (us a call): 1920x1080 of 1M triangles 11,214-11,231 / 11,240 /
+    // 11,584 / 11,238, 2560x1440 19,920-19,965 / 19,990 / 20,528 / 19,961, 1600x900 of 400k 6,058 /
+    // 6,070 / 6,173 / 6,065; 640x360 the same within the runs.
     int thin_from = kThinRound;
     // Whether thin rounds switch for any mix of members (the tuner measured it on the mix)
-    // or only when every member is a large scene (the default: measured faster there, and
-    // slower for small scenes such as the Cornell box).
+    // or only when every member is a large scene (the default: faster there, and slower for
+    // small scenes: the glossy box 3,078 us from round 3 on against 3,005 on the BVH2).
     bool thin_any = false;
     Member *d_members = nullptr;
     unsigned long long *d_stats = nullptr;
@@ -817,9 +820,9 @@ void record_trace(const WaveHost *h, const Wave &w, int width, int stack, int bl
 }
 
 // What a pass's film stage holds besides finish and convert: splats to fold, convergence to
-// check. A launch with nothing to do costs 3 us of a film stage, which the next pass's waits
-// for: without the three, the 256^2 box's four samples take 660 us instead of 688, a 1280x719 view
-// 1,170 instead of 1,193.
+// check. A stage of its own for each, as a launch with nothing to do costs 3 us of a film stage,
+// which the next pass's waits for: with the three idle launches the 256^2 box's four samples take
+// 688 us instead of 660, a 1280x719 view 1,193 instead of 1,170.
 constexpr int kFilmFolds = 1, kFilmAdapts = 2;
 int film_stage(const PlanHeader &head) { return (head.folds ? kFilmFolds : 0) | (head.adapts ? kFilmAdapts : 0); }
 
@@ -1835,9 +1838,9 @@ bool wave_advance(WaveHost *h) {
 // Times two dry passes from the current plan settings (members of size class `only`, or
 // all) and returns their paths a millisecond.
 double time_dry(WaveHost *h, int only, cudaEvent_t a, cudaEvent_t b) {
-    // Warm: builds the variant's graph on every lane. (With one lane warmed, the other's capture
-    // fell between the events, and some variants' rates came out a third of their neighbours';
-    // now they repeat within 2 %.)
+    // Warm: makes the variant's graph on every lane, so that no capture falls between the events
+    // (with one lane warmed some variants' rates came out a third of their neighbours'; with both
+    // they repeat within 2 %).
     for (int i = 0; i < h->lane_count; i++) launch_pass(h, true, only);
     settle(h);
     uint64_t paths = 0;

@@ -48,8 +48,8 @@ __device__ __forceinline__ void write_side(float4 *entries, uint32_t e, uint32_t
 }
 
 // A leaf's box from its triangles' records, which the launch before wrote (they are in L2): three
-// 16-byte loads a triangle, where its indices and points took twelve 4-byte ones (the climb 63 ->
-// 60 us on 1,048,576 triangles: its chain of atomics up the tree is the rest).
+// 16-byte loads a triangle. (From the indices and points, twelve 4-byte loads, the climb takes 63
+// us instead of 60 on 1,048,576 triangles: its chain of atomics up the tree is the rest.)
 __device__ __forceinline__ Box leaf_box(const float4 *tris, int link) {
     const uint32_t code = (uint32_t)(-1 - link);
     const uint32_t first = code >> kLeafShift, count = (code & ((1u << kLeafShift) - 1u)) + 1u;
@@ -208,8 +208,9 @@ __device__ __forceinline__ Box source_box(uint32_t source, const float4 *exact, 
 // box (DeviceWide::boxes) and its bytes of the compressed node, quantized together with the
 // node's other lanes exactly as quantize_node (quantize.hpp) does alone -- the origin and
 // extent by a minimum and a maximum over the lanes, an axis' exponent raised until every lane's
-// planes fit. A thread a node took 111 us on 64,673 nodes (each a loop over 8 x 3 planes, half a
-// wave of threads), half of the refit. Every lane of the warp calls it; `slot` past the end of the tree has none of a node's.
+// planes fit. (A thread a node takes 111 us on 64,673 nodes, each a loop over 8 x 3 planes in half
+// a wave of threads; boxes_kernel is 30 us in all.) Every lane of the warp calls it; a `slot` past
+// the end of the tree has none of a node's.
 __device__ __forceinline__ void wide8_slot(uint64_t slot, bool valid, const uint32_t *sources, const float4 *exact,
                                            const float *root_box, float delta, float4 *nodes, float4 *boxes) {
     constexpr uint32_t kAll = 0xffffffffu;
@@ -276,10 +277,10 @@ __device__ __forceinline__ void wide8_slot(uint64_t slot, bool valid, const uint
 
 // Steps 3 and 4 in one launch, after the climb: the widened BVH2 boxes, the 4-wide tree's and
 // the 8-wide tree's. The widening comes from the new root box on the device, worked out once a
-// block, so nothing waits for the host between the climb and here (which took a copy, a wait and
-// a launch). On 1,048,576 triangles 30 us, latency of the wide slots' scattered box reads for the
-// most part, against 8 + 10 + 111 + 9 in launches of their own; the refit and a query of 32,768
-// rays 314 -> 201 us. The climb is what is left (60 us).
+// block, so nothing waits for the host between the climb and here. On 1,048,576 triangles 30 us,
+// latency of the wide slots' scattered box reads for the most part; in launches of their own
+// 8 + 10 + 111 + 9 and a wait, with which the refit and a query of 32,768 rays take 314 us
+// instead of 201. The climb (59 us) is longer.
 __global__ void __launch_bounds__(256) boxes_kernel(uint64_t entries, float4 *widened, uint64_t slots4, const uint32_t *sources4,
                                                     float4 *nodes4, uint64_t slots8, const uint32_t *sources8,
                                                     float4 *nodes8, float4 *boxes8, const float4 *exact,
