@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kTraceBlockMax, kTraceMinBlocks) closest_kerne
     Visits visits;
     const float4 *ray_o = w.ray_o[q], *ray_d = w.ray_d[q];
     float4 *hits = w.hits[q];
-    typename TracerOf<W, false, kStack, kCount>::type tr(stack + threadIdx.x, blockDim.x);
+    typename TracerOf<W, false, kStack, kCount>::held tr(stack + threadIdx.x, blockDim.x);
     // The camera paths' rays, then the light paths' from the queue's back.
     auto entry = [&](uint32_t j) { return j < cameras ? j : w.pool - 1u - (j - cameras); };
     auto begin = [&](uint32_t j, DeviceScene &s) {
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kTraceBlockMax, kCutouts ? 1 : kTraceMinBlocks
     const uint32_t count = w.counters[w.rounds + 1 + round];
     bool overflow = false;
     Visits visits;
-    typename TracerOf<W, true, kStack, kCount>::type tr(stack + threadIdx.x, blockDim.x);
+    typename TracerOf<W, true, kStack, kCount>::held tr(stack + threadIdx.x, blockDim.x);
     auto member_of = [&](uint32_t tag) -> const Member & { return w.members[w.plan->seg[tag >> kPathBits].member]; };
     auto record = [&](uint32_t i, float state) {
         if (w.record_shadow) w.record_shadow[((size_t)round * w.pool + i) * 3u + 2u] = make_float4(state, 0.0f, 0.0f, 0.0f);
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kTraceBlockMax, kCutouts ? 1 : kTraceMinBlocks
         if (!prologue(i)) return;
         const float4 o = w.shadow_o[i], d = w.shadow_d[i];
         const DeviceScene s = m.scene;
-        typename TracerOf<W, false, kStack, kCount>::type walk(stack + threadIdx.x, blockDim.x);
+        typename TracerOf<W, false, kStack, kCount>::held walk(stack + threadIdx.x, blockDim.x);
         float3 from = xyz(o);
         float remaining = d.w, kept = 1.0f;
         bool through = false;

@@ -93,7 +93,7 @@ __device__ __forceinline__ Hit walk_warp(const DeviceScene &s, const Ray &r, int
                     d = __ldg(tri + 2);
                 }
                 float t, u, v;
-                if (!watertight(sh, r.tmin, limit, a, b, d, t, u, v)) continue;
+                if (!watertight(sh, r.tmin, limit, false, a, b, d, t, u, v)) continue;
                 const int id = __float_as_int(a.w);
                 if (h.id >= 0 && (t > h.t || (t == h.t && id > h.id))) continue;
                 h = Hit{t, id, (int)(first + i), u, v};
