@@ -807,12 +807,12 @@ def main():
     roofline = {
         "kernel": "closest_kernel (intersect closest)",
         # The scene (~100 MB) stays in the 126 MB L2: DRAM moves a few percent of the
-        # algorithmic bytes and is used at 3.6 %, so a fraction of HBM says how fast the
+        # algorithmic bytes and is used at 3.5 %, so a fraction of HBM says how fast the
         # algorithm's bytes are served, not how busy HBM is. Reported against HBM as the
-        # roofline asks; the counters show L1's data pipe at 89 % of its wavefronts on long
+        # roofline asks; the counters show L1's data pipe at 90 % of its wavefronts on long
         # queues (a lane of a divergent load is one), dependent fetches on short ones.
         "bound": "hbm",
-        "bound_observed": "L1 data pipe (long queues; L2-resident scene, HBM at 3.6 %; ncu summary in profiles/)",
+        "bound_observed": "L1 data pipe (long queues; L2-resident scene, HBM at 3.5 %; ncu summary in profiles/)",
         "achieved": achieved,
         "peak": hbm if hbm else 6650.0,
         "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if hbm else "fallback 6.65 TB/s",
